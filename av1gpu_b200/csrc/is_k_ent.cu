@@ -15,10 +15,10 @@
 //   scans         exclusive sums of the blocks' and tx blocks' symbol counts: where each block's and tx block's
 //                 symbols start in the batch's stream, which is in bitstream order
 //   k_ent_emit_*  the symbols into the stream (one thread per block / tx block)
-//   k_ent_code    two warps per tile: the CDF state in shared memory; one warp adapts the CDFs and works out the
-//                 symbols' interval bounds 32 at a time, one lane range-codes the bounds of the batch before, then
-//                 resolves the carries
-//   k_ent_pack    the tiles' payloads back to back, offsets in the result head
+//   k_ent_count .. k_ent_adapt  the CDFs' adaptation over lists of the symbols by CDF; each symbol word becomes the
+//                 range coder's step
+//   k_rg_*        the range coder: the range's course chunk by chunk from every possible start, then the code value as a
+//                 sum of shifted terms with its carries resolved, into the payloads back to back
 // A symbol is one 32-bit word: kind (adaptive / equiprobable bit / split-or-horizontal / split-or-vertical), alphabet
 // size, value and the CDF's offset inside av1g_cdfs.
 #include "is_units.cuh"
@@ -66,9 +66,15 @@ struct EntArgs {
     uint32_t *syms;
     uint64_t cap;
     uint64_t *symBegin;                            // [nTiles + 1]
-    uint16_t *pre;                                 // precarry entries, per tile at 2 * symBegin + 16 * tile
-    uint8_t *tbytes;                               // the tiles' resolved bytes, same places
+    // range coder: chunk starts, start values, the low byte at the end, bits, bits before (per slot), maps (128 bytes a slot), digits (per tile from
+    // symBegin + 16 * tile)
+    uint64_t *rgStart, *rgBit0;
+    uint8_t *rgFirst, *rgLast, *rgMap;
+    uint32_t *rgBits, *rgDigit;
+    uint64_t *tileBits;
     uint32_t *tileBytes;
+    uint32_t *csTab, *csStart, *csLen;             // CDF lists: counts / places per batch slot, start and length per tile
+    uint32_t csPitch;
     is_ent_status *status;
     uint64_t *tileOff;                             // [nTiles + 1], right after the status
     uint8_t *out;
@@ -339,9 +345,12 @@ __device__ void walk_node(Walk &W, int r, int c, int bs) {
     }
 }
 
-__global__ void k_ent_sb(EntArgs A) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= A.nSb) return;
+// One SB a warp, on one lane: the walk is a serial recursion of dependent loads, and 32 of them in a warp take turns (a
+// thread per SB, 64 a CTA: 2.95 ms for the 12 MP picture's 2961 SBs).
+constexpr int SB_WARPS = 4;
+__global__ void __launch_bounds__(SB_WARPS * 32) k_ent_sb(EntArgs A) {
+    const uint32_t g = blockIdx.x * SB_WARPS + (threadIdx.x >> 5);
+    if (g >= A.nSb || (threadIdx.x & 31)) return;
     const EntFrameD &F = A.fr[ent_find(A.fSb, A.nF, g)];
     const int s = (int)(g - F.sbBase), sr = s / F.sbCols, sc = s - sr * F.sbCols;
     Walk W;
@@ -592,215 +601,647 @@ __global__ void k_ent_emit_txb(EntArgs A) {
     if (S.n != cnt) ent_fail(A, IS_ENT_ERR_RECORD);
 }
 
-// ---- the range coder: AV1's multi-symbol arithmetic coder (spec 8.2.6 read_symbol, from the encoder's side; the
-// interval split (15-bit probabilities, 4 per symbol reserved), renormalisation and flush follow libaom's
-// od_ec_encode_q15 / od_ec_enc_done, which the decoder's arithmetic fixes to the bit).  Output goes to a precarry buffer of 16-bit entries (a byte plus a possible carry);
-// the carries are resolved backwards when the tile is done. ----
-struct RangeEnc {
-    uint32_t low, rng;
-    int cnt;           // bits of low waiting below the next output byte, minus 16 (starts at -9)
-    uint32_t n, cap;
-    uint16_t *pre;
-    bool over;
-    __device__ void init(uint16_t *p, uint32_t c) { low = 0; rng = 0x8000; cnt = -9; n = 0; cap = c; pre = p; over = false; }
-    __device__ __forceinline__ void out(uint32_t v) {
-        if (n < cap) pre[n] = (uint16_t)v; else over = true;
-        n++;
-    }
-    // one symbol from its packed step (pack_step): the interval split of the symbol, then renormalisation of the range
-    // to 16 bits, where every 8 bits of low that pass the window go out.  The arithmetic chain through the range is
-    // kept short: the probability terms come precomputed.
-    __device__ __forceinline__ void step(uint32_t e) {
-        const uint32_t r = rng, r8 = r >> 8;
-        const uint32_t ev = (e >> 20) & 63u;
-        const uint32_t v = ((r8 * ((e >> 10) & 0x3FFu)) >> 1) + ev;
-        const uint32_t u = (e >> 26) ? r : ((r8 * (e & 0x3FFu)) >> 1) + ev + 4u;
-        uint32_t l = low + (r - u);
-        const uint32_t rn = u - v;
-        const int d = __clz(rn) - 16;
-        int s = cnt + d;
-        if (s >= 0) {
-            int c = cnt + 16;
-            const int bytes = s >= 8 ? 2 : 1;
-            for (int i = 0; i < bytes; i++) {
-                out(l >> c);
-                l &= (1u << c) - 1;
-                c -= 8;
-            }
-            s = c + d - 16;
-        }
-        low = l << d;
-        rng = rn << d;
-        cnt = s;
-    }
-    // flush: the shortest tail that keeps the final interval decodable, then the carries; returns the byte count
-    __device__ uint32_t finish(uint8_t *bytes) {
-        uint32_t e = ((low + 0x3FFFu) & ~0x3FFFu) | 0x4000u;
-        int c = cnt, s = c + 10;
-        if (s > 0) {
-            uint32_t m = (1u << (c + 16)) - 1;
-            do {
-                out(e >> (c + 16));
-                e &= m;
-                s -= 8;
-                c -= 8;
-                m >>= 8;
-            } while (s > 0);
-        }
-        if (over) return 0;
-        uint32_t carry = 0;
-        for (uint32_t i = n; i-- > 0;) {
-            carry += pre[i];
-            bytes[i] = (uint8_t)carry;
-            carry >>= 8;
-        }
-        return n;
-    }
-};
-// the coder's inputs of symbol s of an alphabet of nm1 + 1 symbols with bounds fl / fh (32768 x the probability of the
-// symbols after s - 1 / after s): fl >> 6, fh >> 6, 4 (nm1 - s), and whether fl is the whole range
-__device__ __forceinline__ uint32_t pack_step(uint32_t fl, uint32_t fh, int s, int nm1) {
-    return (fl >> 6) | ((fh >> 6) << 10) | ((uint32_t)(4 * (nm1 - s)) << 20) | ((fl >= 32768u ? 1u : 0u) << 26);
-}
+// ---- CDF adaptation: the symbols' interval bounds ----
+// A coder step of symbol s of an alphabet of nm1 + 1 symbols with bounds fl / fh (32768 x the probability of the
+// symbols after s - 1 / after s): the upper half holds fl's bits from 6 on (the coder reads no lower ones; bit 15 set: fl
+// is the whole range, symbol 0) and nm1 - s below them, the lower half fh
+__device__ __forceinline__ uint32_t step_hi(uint32_t fl, int below) { return (fl & 0xFFC0u) | (uint32_t)below; }
+__device__ __forceinline__ uint32_t pack_step(uint32_t fl, uint32_t fh, int s, int nm1) { return (step_hi(fl, nm1 - s) << 16) | fh; }
+constexpr uint32_t STEP_FIRST = 1u << 31;
+__device__ __forceinline__ uint32_t step_ev(uint32_t e) { return (e >> 14) & 0xFCu; }   // 4 (nm1 - s)
 
-// CDF adaptation (spec 8.2.6 symbol decoding process, disable_cdf_update 0): spec-format CDF (cumulative, last
-// entry 32768) followed by its counter
-__device__ __forceinline__ void adapt(uint16_t *cdf, int s, int N) {
-    const int count = cdf[N];
-    const int rate = 3 + (count > 15) + (count > 31) + (N > 3 ? 2 : 1);
-    for (int i = 0; i < N - 1; i++) {
-        const int v = cdf[i];
-        cdf[i] = (uint16_t)(i < s ? v - (v >> rate) : v + ((32768 - v) >> rate));
-    }
-    cdf[N] = (uint16_t)(count + (count < 32));
-}
+// the CDFs the symbols use, numbered: CDF i starts at entry g_cdfOff[i] of av1g_cdfs and has g_cdfN[i] symbols;
+// g_cdfId[offset / 3] is its number (distinct CDFs start at least 3 entries apart)
+constexpr int NID_MAX = 1536;
+static __device__ uint16_t g_cdfId[NCDF / 3 + 1];
+static __device__ uint16_t g_cdfOff[NID_MAX];
+static __device__ uint8_t g_cdfN[NID_MAX];
+static __device__ uint16_t g_cdfOrder[NID_MAX];   // the CDFs of up to 4 symbols, then the larger ones
+static __constant__ int c_nCdf;
 
 // the probability mass of the partitions that split the bottom half (split_or_horz) or the right half
-// (split_or_vert) of a node at the frame edge (spec 9.3.1, split_or_horz / split_or_vert cdf)
-__device__ __forceinline__ uint32_t split_mass(const uint16_t *pc, bool vert) {
-    auto P = [&](int x) { return (uint32_t)pc[x] - (x ? (uint32_t)pc[x - 1] : 0u); };
-    return vert ? P(AV1G_PARTITION_HORZ) + P(AV1G_PARTITION_SPLIT) + P(AV1G_PARTITION_HORZ_A) + P(AV1G_PARTITION_HORZ_B) +
-                      P(AV1G_PARTITION_VERT_A) + P(AV1G_PARTITION_HORZ_4)
-                : P(AV1G_PARTITION_VERT) + P(AV1G_PARTITION_SPLIT) + P(AV1G_PARTITION_HORZ_A) + P(AV1G_PARTITION_VERT_A) +
-                      P(AV1G_PARTITION_VERT_B) + P(AV1G_PARTITION_VERT_4);
+// (split_or_vert) of a node at the frame edge (spec 9.3.1, split_or_horz / split_or_vert cdf), as a bit set
+__device__ __forceinline__ uint32_t split_set(bool vert) {
+    return vert ? (1u << AV1G_PARTITION_HORZ) | (1u << AV1G_PARTITION_SPLIT) | (1u << AV1G_PARTITION_HORZ_A) | (1u << AV1G_PARTITION_HORZ_B) |
+                      (1u << AV1G_PARTITION_VERT_A) | (1u << AV1G_PARTITION_HORZ_4)
+                : (1u << AV1G_PARTITION_VERT) | (1u << AV1G_PARTITION_SPLIT) | (1u << AV1G_PARTITION_HORZ_A) | (1u << AV1G_PARTITION_VERT_A) |
+                      (1u << AV1G_PARTITION_VERT_B) | (1u << AV1G_PARTITION_VERT_4);
 }
 
-// Two warps per tile.  Warp 0 turns the symbols into coder inputs 32 at a time: a symbol's interval bounds (fl, fh)
-// depend on its CDF as the earlier symbols left it, so the symbols of a window that share a CDF form a group (lanes
-// with equal CDF offsets) whose lowest lane walks them in order, adapting the CDF - in registers for alphabets of up
-// to 4 symbols (the coefficient CDFs, which carry long runs), in shared memory otherwise; groups and the equiprobable
-// bits proceed side by side; each symbol leaves its coder step (pack_step).  Lane 0 of warp 1 runs only the range
-// coder's arithmetic over the previous batch of steps, so the two overlap batch by batch.
-constexpr int CODE_BATCH = 1024;   // symbols per batch (a multiple of 32)
-
-// the coder step of symbol s of a CDF of up to 4 symbols held as c0..c2 (the last entry is 32768), then its adaptation
-__device__ __forceinline__ uint32_t bounds_small(uint32_t c[3], uint32_t &count, int s, int N) {
-    const uint32_t cs = s == 0 ? c[0] : s == 1 ? (N > 2 ? c[1] : 32768u) : s == 2 ? (N > 3 ? c[2] : 32768u) : 32768u;
-    const uint32_t cp = s == 1 ? c[0] : s == 2 ? c[1] : c[2];
-    const uint32_t fl = s ? 32768u - cp : 32768u, fh = 32768u - cs;
-    const int rate = 3 + (count > 15) + (count > 31) + (N > 3 ? 2 : 1);
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-        if (i < N - 1) c[i] = i < s ? c[i] - (c[i] >> rate) : c[i] + ((32768u - c[i]) >> rate);
-    count += count < 32;
-    return pack_step(fl, fh, s, N - 1);
+// A symbol's bounds depend on its CDF as the earlier symbols of that CDF left it and on nothing else: the symbols of a
+// tile are sorted by CDF, stably, and the lists are walked side by side over the whole GPU.
+//   k_ent_count    batches of CS_B symbols: how many symbols each CDF has in the batch
+//   k_ent_place    per tile: where each CDF's list starts, and each batch's part in it
+//   k_ent_scatter  batches again: the symbols to their places in the lists (each warp ranks its 256 symbols against
+//                  per-warp counters); the equiprobable bits, which have no CDF, to coder steps at once
+//   k_ent_adapt    the lists: 4 lanes per CDF of up to 4 symbols (the coefficient CDFs, which carry the long lists), 16 per
+//                  larger CDF; each symbol word becomes its coder step
+// What bounds it is the longest list of a tile (about 7 % of its symbols): a serial chain of one step a symbol.  The 12 MP
+// picture's two tiles: 10.1 ms for the four kernels, where two warps per tile that adapted 32 symbols at a time and
+// range-coded them on one lane took 400 ms.
+constexpr int CS_T = 512, CS_WARPS = CS_T / 32, CS_SEG = 256, CS_B = CS_WARPS * CS_SEG, CS_PAD = 24;
+struct CsSmem {
+    uint16_t cnt[NID_MAX][CS_PAD];         // per CDF and warp: symbols, then the warps before (rows of 48 bytes: eight
+                                           // lanes' 16-byte loads meet no common bank)
+    uint16_t id[NCDF / 3 + 2];
+};
+static_assert(sizeof(CsSmem) <= 113 * 1024, "k_ent_scatter: two CTAs per SM");
+// batch slots: tile t's batch k is slot symBegin[t] / CS_B + t + k
+__device__ __forceinline__ uint64_t cs_slot0(const EntArgs &A, uint32_t t) { return A.symBegin[t] / CS_B + t; }
+__device__ __forceinline__ uint32_t cs_batches(const EntArgs &A, uint32_t t) {
+    return (uint32_t)((A.symBegin[t + 1] - A.symBegin[t] + CS_B - 1) / CS_B);
 }
-
-__global__ void __launch_bounds__(64) k_ent_code(EntArgs A) {
-    __shared__ __align__(16) uint16_t cdf[NCDF];
-    __shared__ uint32_t bnd[2][CODE_BATCH];   // the coder steps (pack_step)
-    __shared__ uint32_t words[CODE_BATCH];    // warp 0's batch of symbol words
-    const uint32_t g = blockIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (A.status->error) return;
-    const EntFrameD &F = A.fr[ent_find(A.fTile, A.nF, g)];
-    {
-        const uint4 *src = reinterpret_cast<const uint4 *>(g_cdfInit[F.qctx]);
-        for (int i = threadIdx.x; i < NCDF / 8; i += 64) reinterpret_cast<uint4 *>(cdf)[i] = src[i];
+__device__ __forceinline__ bool cs_find(const EntArgs &A, uint64_t slot, uint32_t &t, uint32_t &k) {
+    uint32_t lo = 0, hi = A.nTiles - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (cs_slot0(A, mid) <= slot) lo = mid; else hi = mid - 1;
     }
-    const uint64_t s0 = A.symBegin[g], s1 = A.symBegin[g + 1];
-    const uint64_t base = 2 * s0 + 16 * (uint64_t)g;
-    const uint32_t nb = (uint32_t)((s1 - s0 + CODE_BATCH - 1) / CODE_BATCH);
-    RangeEnc E;
-    E.init(A.pre + base, (uint32_t)(2 * (s1 - s0) + 16));
-    __syncthreads();
-    for (uint32_t b = 0; b <= nb; b++) {
-        if (warp == 0 && b < nb) {
-            const uint64_t at = s0 + (uint64_t)b * CODE_BATCH;
-            const int n = (int)min((uint64_t)CODE_BATCH, s1 - at);
-            uint32_t *pb = bnd[b & 1];
-#pragma unroll 8
-            for (int j = lane; j < n; j += 32) words[j] = A.syms[at + j];   // the batch's loads in flight together
-            __syncwarp();
-            for (int j = 0; j < n; j += 32) {
-                const bool live = j + lane < n;
-                const uint32_t w = live ? words[j + lane] : (uint32_t)SYM_BIT;
-                const int kind = w & 3, nm1 = (w >> 2) & 15, s = (w >> 6) & 15;
-                const uint32_t key = kind == SYM_BIT ? 0x80000000u | lane : (w >> 16);
-                const uint32_t same = __match_any_sync(0xffffffffu, key);
-                if (live) {
-                    if (kind == SYM_BIT) {
-                        pb[j + lane] = pack_step(s ? 16384u : 32768u, s ? 0u : 16384u, s, 1);
-                    } else if (lane == __ffs(same) - 1) {   // the group's leader walks its members in order
-                        uint16_t *c = cdf + (w >> 16);
-                        const uint32_t m = same;   // only live lanes carry CDF keys
-                        bool small = kind == SYM_ADAPT && nm1 < 4;
-                        for (uint32_t t = m; t && small; t &= t - 1) small = (words[j + __ffs(t) - 1] & 3) == SYM_ADAPT;
-                        if (small) {
-                            const int N = nm1 + 1;
-                            uint32_t cv[3] = {c[0], N > 2 ? c[1] : 0u, N > 3 ? c[2] : 0u};
-                            uint32_t count = c[N];
-                            int k = j + __ffs(m) - 1;
-                            uint32_t wk = words[k];
-                            for (uint32_t t = m; t;) {   // the next member's word is loaded while this one is coded
-                                const uint32_t tn = t & (t - 1);
-                                const int kn = tn ? j + __ffs(tn) - 1 : k;
-                                const uint32_t wn = words[kn];
-                                pb[k] = bounds_small(cv, count, (wk >> 6) & 15, N);
-                                t = tn;
-                                k = kn;
-                                wk = wn;
-                            }
-                            c[0] = (uint16_t)cv[0];
-                            if (N > 2) c[1] = (uint16_t)cv[1];
-                            if (N > 3) c[2] = (uint16_t)cv[2];
-                            c[N] = (uint16_t)count;
-                        } else {
-                            for (uint32_t t = m; t; t &= t - 1) {
-                                const int k = j + __ffs(t) - 1;
-                                const uint32_t wk = words[k];
-                                const int kk = wk & 3, nk = (wk >> 2) & 15, sk = (wk >> 6) & 15;
-                                uint32_t fl, fh;
-                                if (kk == SYM_ADAPT) {
-                                    fl = sk ? 32768u - c[sk - 1] : 32768u;
-                                    fh = 32768u - c[sk];
-                                    adapt(c, sk, nk + 1);
-                                } else {
-                                    const uint32_t ms = split_mass(c, kk == SYM_SPLIT_V);
-                                    fl = sk ? ms : 32768u;
-                                    fh = sk ? 0u : ms;
-                                }
-                                pb[k] = pack_step(fl, fh, sk, nk);
-                            }
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        if (warp == 1 && lane == 0 && b > 0) {
-            const uint64_t at = s0 + (uint64_t)(b - 1) * CODE_BATCH;
-            const int n = (int)min((uint64_t)CODE_BATCH, s1 - at);
-            const uint32_t *pb = bnd[(b - 1) & 1];
-#pragma unroll 4
-            for (int j = 0; j < n; j++) E.step(pb[j]);
+    t = lo;
+    k = (uint32_t)(slot - cs_slot0(A, lo));
+    return k < cs_batches(A, lo);
+}
+__device__ __forceinline__ uint64_t cs_slots(const EntArgs &A) { return A.symBegin[A.nTiles] / CS_B + A.nTiles; }
+// the table of a slot's counts, then list places; a tile's lists lie where its digits will be
+__device__ __forceinline__ uint32_t *cs_row(const EntArgs &A, uint64_t slot) { return A.csTab + slot * A.csPitch; }
+__device__ __forceinline__ uint32_t *cs_lists(const EntArgs &A, uint32_t t) { return A.rgDigit + A.symBegin[t] + 16 * (uint64_t)t; }
+
+__global__ void __launch_bounds__(CS_T) k_ent_count(EntArgs A) {
+    __shared__ uint32_t hist[NID_MAX];
+    __shared__ uint16_t sid[NCDF / 3 + 1];
+    if (A.status->error) return;
+    const int nId = c_nCdf, tid = threadIdx.x;
+    for (int i = tid; i < NCDF / 3 + 1; i += CS_T) sid[i] = g_cdfId[i];
+    const uint64_t ns = cs_slots(A);
+    for (uint64_t slot = blockIdx.x; slot < ns; slot += gridDim.x) {
+        uint32_t t, k;
+        if (!cs_find(A, slot, t, k)) continue;
+        const uint64_t at = A.symBegin[t] + (uint64_t)k * CS_B;
+        const int n = (int)min((uint64_t)CS_B, A.symBegin[t + 1] - at);
+        __syncthreads();
+        for (int i = tid; i < nId; i += CS_T) hist[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < CS_B / CS_T; q++) {
+            const int i = q * CS_T + tid;
+            const uint32_t w = i < n ? A.syms[at + i] : (uint32_t)SYM_BIT;
+            if ((w & 3) != SYM_BIT) atomicAdd(&hist[sid[(w >> 16) / 3]], 1u);
         }
         __syncthreads();
+        uint32_t *row = cs_row(A, slot);
+        for (int i = tid; i < nId; i += CS_T) row[i] = hist[i];
     }
-    if (warp == 1 && lane == 0) {
-        const uint32_t bytes = E.finish(A.tbytes + base);
-        if (E.over) ent_fail(A, IS_ENT_ERR_OUTPUT);
-        A.tileBytes[g] = bytes;
+}
+
+__global__ void __launch_bounds__(SCAN_T) k_ent_place(EntArgs A) {
+    __shared__ uint32_t sh[32];
+    if (A.status->error) return;
+    const uint32_t t = blockIdx.x, nb = cs_batches(A, t);
+    const int nId = c_nCdf;
+    uint32_t *row0 = cs_row(A, cs_slot0(A, t));
+    uint32_t carry = 0;
+    for (int id0 = 0; id0 < nId; id0 += SCAN_T) {
+        const int id = id0 + threadIdx.x;
+        uint32_t run = 0;
+        if (id < nId) {
+            uint32_t *p = row0 + id;
+            uint32_t b = 0;
+            for (; b + 8 <= nb; b += 8) {
+                uint32_t v[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] = p[(uint64_t)(b + i) * A.csPitch];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    p[(uint64_t)(b + i) * A.csPitch] = run;
+                    run += v[i];
+                }
+            }
+            for (; b < nb; b++) {
+                const uint32_t v = p[(uint64_t)b * A.csPitch];
+                p[(uint64_t)b * A.csPitch] = run;
+                run += v;
+            }
+        }
+        uint32_t tot;
+        const uint32_t e = cta_exclusive(run, sh, &tot);
+        if (id < nId) {
+            A.csStart[(uint64_t)t * A.csPitch + id] = carry + e;
+            A.csLen[(uint64_t)t * A.csPitch + id] = run;
+        }
+        carry += tot;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(CS_T) k_ent_scatter(EntArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CsSmem &S = *reinterpret_cast<CsSmem *>(smem_raw);
+    if (A.status->error) return;
+    const int nId = c_nCdf, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < NCDF / 3 + 1; i += CS_T) S.id[i] = g_cdfId[i];
+    const uint64_t ns = cs_slots(A);
+    for (uint64_t slot = blockIdx.x; slot < ns; slot += gridDim.x) {
+        uint32_t t, k;
+        if (!cs_find(A, slot, t, k)) continue;
+        const uint64_t at = A.symBegin[t] + (uint64_t)k * CS_B;
+        const int n = (int)min((uint64_t)CS_B, A.symBegin[t + 1] - at);
+        __syncthreads();
+        for (int i = tid; i < nId * (CS_PAD / 8); i += CS_T) reinterpret_cast<uint4 *>(S.cnt)[i] = make_uint4(0, 0, 0, 0);
+        uint32_t word[CS_SEG / 32], mine[CS_SEG / 32];   // CDF number | rank among the warp's << 16; NONE32: no CDF
+#pragma unroll
+        for (int q = 0; q < CS_SEG / 32; q++) {
+            const int i = warp * CS_SEG + q * 32 + lane;
+            word[q] = i < n ? A.syms[at + i] : (uint32_t)SYM_BIT;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < CS_SEG / 32; q++) {
+            const uint32_t w = word[q];
+            const bool has = (w & 3) != SYM_BIT;
+            const uint32_t id = has ? S.id[(w >> 16) / 3] : 0x10000u + lane;
+            const uint32_t same = __match_any_sync(0xffffffffu, id);
+            uint32_t before = 0;
+            if (has) before = S.cnt[id][warp];
+            mine[q] = has ? id | ((before + __popc(same & ((1u << lane) - 1))) << 16) : NONE32;
+            __syncwarp();
+            if (has && lane == __ffs(same) - 1) S.cnt[id][warp] = (uint16_t)(before + __popc(same));
+            __syncwarp();
+        }
+        __syncthreads();
+        for (int id = tid; id < nId; id += CS_T) {   // the warps' counts to the symbols of the warps before
+            uint4 *row = reinterpret_cast<uint4 *>(S.cnt[id]);
+            uint32_t run = 0;
+#pragma unroll
+            for (int q = 0; q < CS_WARPS / 8; q++) {
+                const uint4 v = row[q];
+                const uint32_t c[4] = {v.x, v.y, v.z, v.w};
+                uint32_t o[4];
+#pragma unroll
+                for (int z = 0; z < 4; z++) {
+                    const uint32_t lo = c[z] & 0xFFFFu, hi = c[z] >> 16;
+                    o[z] = run | ((run + lo) << 16);
+                    run += lo + hi;
+                }
+                row[q] = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        }
+        __syncthreads();
+        const uint32_t *row = cs_row(A, slot), *start = A.csStart + (uint64_t)t * A.csPitch;
+        uint32_t *lists = cs_lists(A, t);
+#pragma unroll
+        for (int q = 0; q < CS_SEG / 32; q++) {
+            const int i = warp * CS_SEG + q * 32 + lane;
+            if (i >= n) continue;
+            const uint32_t w = word[q], s = (w >> 6) & 15;
+            if (mine[q] == NONE32) {
+                A.syms[at + i] = pack_step(s ? 16384u : 32768u, s ? 0u : 16384u, (int)s, 1);
+            } else {
+                // an entry: the symbol's index in its tile, and for an alphabet of up to 4 the symbol in the upper 2
+                // bits (a tile of at most 4096 x 2304 samples has fewer than 2^30 symbols)
+                const uint32_t id = mine[q] & 0xFFFFu, ix = k * (uint32_t)CS_B + i;
+                lists[start[id] + row[id] + S.cnt[id][warp] + (mine[q] >> 16)] = g_cdfN[id] > 4 ? ix : ix | (s << 30);
+            }
+        }
+    }
+}
+
+// The CDFs in the inverse form of the bounds, a = 32768 - c: symbol s has fl = a[s - 1] (32768 for s = 0) and fh = a[s] (0
+// for the last); spec 8.2.6's adaptation moves entries before s up by (32768 - a) >> rate and the others down by
+// a >> rate, which is a += (T - a) >> rate with T = 32768 or 2^rate - 1 (the arithmetic shift rounds down).
+// A lane holds one entry a: 4 lanes walk a CDF of up to 4 symbols, 16 a larger one.  The lane of entry s leaves the
+// step's lower half, that of entry s - 1 the upper one (the last lane for s = 0), so a symbol costs no exchange between
+// lanes.  One lane with the three entries of a small CDF, the bounds selected and packed, took 100 cycles a symbol.
+__device__ __forceinline__ void adapt_entry(int &a, int j, int s, int nm1, int last, int rate, uint16_t *at) {
+    const int up = s > j;
+    if (j == s) at[0] = (uint16_t)a;
+    if (s ? j == s - 1 : j == last) at[1] = (uint16_t)step_hi(s ? (uint32_t)a : 32768u, nm1 - s);
+    a += ((up ? 32768 : (1 << rate) - 1) - a) >> rate;
+}
+__global__ void __launch_bounds__(32) k_ent_adapt(EntArgs A, int smallWarps, int nSmall, int nLarge, int warpsPerTile) {
+    if (A.status->error) return;
+    const uint32_t t = blockIdx.x / warpsPerTile;
+    const int part = (int)(blockIdx.x % warpsPerTile), lane = threadIdx.x;
+    const EntFrameD &F = A.fr[ent_find(A.fTile, A.nF, t)];
+    const uint16_t *init = g_cdfInit[F.qctx];
+    const uint32_t *lists = cs_lists(A, t);
+    const uint32_t *start = A.csStart + (uint64_t)t * A.csPitch, *lens = A.csLen + (uint64_t)t * A.csPitch;
+    uint32_t *sym = A.syms + A.symBegin[t];
+    uint16_t *step = reinterpret_cast<uint16_t *>(sym);
+    if (part < smallWarps) {
+        const int l = part * 8 + (lane >> 2), j = lane & 3;
+        if (l >= nSmall) return;
+        const int id = g_cdfOrder[l], nm1 = g_cdfN[id] - 1;
+        const uint32_t m = lens[id];
+        const uint16_t *c = init + g_cdfOff[id];
+        const uint32_t *q = lists + start[id];
+        int a = j < nm1 ? 32768 - c[j] : 0;   // the last entry, and those a shorter alphabet has not, stay 0: s is below them
+        const int e = nm1 > 2 ? 5 : 4;
+        auto one = [&](uint32_t w, int rate) { adapt_entry(a, j, (int)(w >> 30), nm1, 3, rate, step + 2 * (uint64_t)(w & 0x3FFFFFFFu)); };
+        uint32_t k = 0;
+        const uint32_t count = c[nm1 + 1];
+        // the first 32 symbols adapt faster; then up to the first 16-byte boundary of the list
+        for (; k < m && (k + count < 32 || ((uintptr_t)(q + k) & 15)); k++) one(q[k], e + (k + count > 15) + (k + count > 31));
+        const int rate = e + 2;
+        auto load = [&](uint32_t at) { return at + 4 <= m ? *reinterpret_cast<const uint4 *>(q + at) : make_uint4(0, 0, 0, 0); };
+        uint4 n0 = load(k), n1 = load(k + 4);
+        for (; k + 8 <= m; k += 8) {   // the entries are loaded 8 ahead of their use
+            const uint4 v0 = n0, v1 = n1;
+            n0 = load(k + 8);
+            n1 = load(k + 12);
+            one(v0.x, rate); one(v0.y, rate); one(v0.z, rate); one(v0.w, rate);
+            one(v1.x, rate); one(v1.y, rate); one(v1.z, rate); one(v1.w, rate);
+        }
+        for (; k < m; k++) one(q[k], rate);
+    } else {
+        const int half = lane >> 4, j = lane & 15, l = (part - smallWarps) * 2 + half;
+        const bool on = l < nLarge;
+        const int id = g_cdfOrder[nSmall + (on ? l : 0)], nm1 = g_cdfN[id] - 1;
+        const uint32_t m = on ? lens[id] : 0;
+        const uint16_t *c = init + g_cdfOff[id];
+        const uint32_t *q = lists + start[id];
+        int a = j < nm1 ? 32768 - c[j] : 0;
+        const uint32_t mm = max(m, __shfl_xor_sync(0xffffffffu, m, 16));   // both halves go through the same steps
+        uint32_t count = c[nm1 + 1];
+        // entries two groups of 4 ahead, their symbol words one group ahead
+        uint32_t ix[4], ixn[4], w[4], wn[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            ix[i] = i < m ? q[i] : 0u;
+            ixn[i] = 4 + i < m ? q[4 + i] : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) w[i] = i < m ? sym[ix[i]] : 0u;
+        for (uint32_t k0 = 0; k0 < mm; k0 += 4) {
+            uint32_t ixf[4];
+            bool edge = false;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                wn[i] = k0 + 4 + i < m ? sym[ixn[i]] : 0u;
+                ixf[i] = k0 + 8 + i < m ? q[k0 + 8 + i] : 0u;
+                edge |= (w[i] & 3) != SYM_ADAPT;
+            }
+            edge = __any_sync(0xffffffffu, edge);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t k = k0 + i;
+                const int s = (int)(w[i] >> 6) & 15, kind = w[i] & 3;
+                if (edge) {   // a node at the frame edge: its partitions' mass, no adaptation
+                    int below = __shfl_up_sync(0xffffffffu, a, 1, 16);
+                    if (j == 0) below = 32768;
+                    uint32_t mass = (split_set(kind == SYM_SPLIT_V) >> j) & 1 ? (uint32_t)(below - a) : 0u;
+                    for (int o = 8; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+                    if (k < m && kind != SYM_ADAPT) {
+                        if (j == 0) sym[ix[i]] = pack_step(s ? mass : 32768u, s ? 0u : mass, s, 1);
+                        continue;
+                    }
+                }
+                if (k < m) adapt_entry(a, j, s, nm1, 15, 5 + (count > 15) + (count > 31), step + 2 * (uint64_t)ix[i]);
+                count++;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) { ix[i] = ixn[i]; w[i] = wn[i]; ixn[i] = ixf[i]; }
+        }
+    }
+}
+
+// ---- the range coder: AV1's multi-symbol arithmetic coder (spec 8.2.6 read_symbol, from the encoder's side; the
+// interval split (15-bit probabilities, 4 per symbol reserved), renormalisation and flush follow libaom's
+// od_ec_encode_q15 / od_ec_enc_done, which the decoder's arithmetic fixes to the bit).
+//
+// The coder's state is the range r (32768 .. 65535) and the code value.  The value never feeds back into the range, so
+// a tile is coded in parallel:
+//   the range     a step reads r only through r >> 8, except a step of symbol 0 (STEP_FIRST), which keeps r - v.  So
+//                 from a step that is not one, the range takes one of 128 courses: k_rg_map runs a chunk of steps from
+//                 each of the 128 values (one lane each) to the value it ends with, k_rg_chain strings the chunks' maps
+//                 together, and k_rg_walk runs every chunk once more from the value it starts with.  128 times the
+//                 work, but on 128 times the lanes: 1.9 ms for the 12 MP picture (k_rg_map 0.74, the others below 0.5 each).
+//   the value     is the sum over the steps of (r - u) 2^-(bits the steps before shifted out): k_rg_bits adds the terms
+//                 into 16-bit digits (held in 32 bits) at their places, k_rg_carry carries them through.
+constexpr int RG_CH = 1024;            // steps per chunk (nominal: a chunk starts at the first step from there that is
+                                       // not a STEP_FIRST; a stretch without one belongs to the chunk before)
+constexpr int RG_STATES = 128;
+
+// one range step in a form with a short dependent chain.  The range is held as the float bits of the unnormalised
+// range: its mantissa is the normalised one, so the renormalisation is an addition (the magic-number conversion of the
+// 16-bit sum), and (r >> 8) in bits 16-23 gives ((r >> 8) p) >> 1 as the upper word of one product with p << 15.
+struct RangeStep {
+    uint32_t mu, mv, keep, k;          // p of fl and fh << 15 (0 for fl of a STEP_FIRST); 0xFFFF for a STEP_FIRST; the rest
+};
+__device__ __forceinline__ RangeStep range_step(uint32_t e) {
+    const bool first = e & STEP_FIRST;
+    RangeStep s;
+    s.mu = first ? 0u : (e & 0xFFC00000u) >> 7;
+    s.mv = (e & 0xFFC0u) << 9;
+    s.keep = first ? 0xFFFFu : 0u;
+    s.k = 0x4B000000u + (first ? 0u - step_ev(e) : 4u);
+    return s;
+}
+__device__ __forceinline__ uint32_t range_bits(uint32_t r) { return __float_as_uint((float)r); }
+__device__ __forceinline__ uint32_t range_of(uint32_t b) { return ((b >> 8) & 0x7FFFu) | 0x8000u; }   // the normalised range
+__device__ __forceinline__ uint32_t range_next(uint32_t b, const RangeStep &s) {   // float bits of u - v
+    const uint32_t r8 = (b & 0x7F0000u) | 0x800000u;
+    const uint32_t rn = (__umulhi(r8, s.mu) + s.k) - __umulhi(r8, s.mv) + (range_of(b) & s.keep);
+    return __float_as_uint(__uint_as_float(rn) - 8388608.0f);
+}
+
+// chunk slots: tile t's chunk k is slot symBegin[t] / RG_CH + t + k
+__device__ __forceinline__ uint64_t rg_slot0(const EntArgs &A, uint32_t t) { return A.symBegin[t] / RG_CH + t; }
+__device__ __forceinline__ uint32_t rg_chunks(const EntArgs &A, uint32_t t) {
+    return (uint32_t)((A.symBegin[t + 1] - A.symBegin[t] + RG_CH - 1) / RG_CH);
+}
+// the tile of a slot, and its chunk number; false for a slot that no chunk has
+__device__ __forceinline__ bool rg_find(const EntArgs &A, uint64_t slot, uint32_t &t, uint32_t &k) {
+    uint32_t lo = 0, hi = A.nTiles - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (rg_slot0(A, mid) <= slot) lo = mid; else hi = mid - 1;
+    }
+    t = lo;
+    k = (uint32_t)(slot - rg_slot0(A, lo));
+    return k < rg_chunks(A, lo);
+}
+__device__ __forceinline__ uint64_t rg_slots(const EntArgs &A) { return A.symBegin[A.nTiles] / RG_CH + A.nTiles; }
+
+// where each chunk starts (NONE: the stretch has no step to start from)
+__global__ void k_rg_starts(EntArgs A) {
+    if (A.status->error) return;
+    const uint64_t ns = rg_slots(A);
+    for (uint64_t slot = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; slot < ns; slot += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t t, k;
+        uint64_t at = ~0ull;
+        if (rg_find(A, slot, t, k)) {
+            const uint64_t j0 = A.symBegin[t] + (uint64_t)k * RG_CH, j1 = min(j0 + RG_CH, A.symBegin[t + 1]);
+            if (k == 0) at = j0;
+            else
+                for (uint64_t j = j0; j < j1; j++)
+                    if (!(A.syms[j] & STEP_FIRST)) { at = j; break; }
+        }
+        A.rgStart[slot] = at;
+    }
+}
+// the end of a chunk: the start of the next chunk of its tile that has one, or the tile's end
+__device__ __forceinline__ uint64_t rg_end(const EntArgs &A, uint64_t slot, uint32_t t, uint32_t k) {
+    const uint32_t nc = rg_chunks(A, t);
+    for (uint32_t q = 1; k + q < nc; q++) {
+        const uint64_t at = A.rgStart[slot + q];
+        if (at != ~0ull) return at;
+    }
+    return A.symBegin[t + 1];
+}
+
+// the map of each chunk: start value r >> 8 (one lane each; the tile's first chunk starts at r = 32768) to end value.
+// Two operations on memory a step (one broadcast 16-byte load), about 12 on the ALUs: bound by issue, 148 SMs share it.
+__global__ void __launch_bounds__(RG_STATES) k_rg_map(EntArgs A) {
+    __shared__ uint4 st[256];
+    if (A.status->error) return;
+    const uint64_t ns = rg_slots(A);
+    const int tid = threadIdx.x;
+    for (uint64_t slot = blockIdx.x; slot < ns; slot += gridDim.x) {
+        uint32_t t, k;
+        const uint64_t at = A.rgStart[slot];
+        if (at == ~0ull) continue;
+        rg_find(A, slot, t, k);
+        const uint64_t end = rg_end(A, slot, t, k);
+        uint32_t b = range_bits(k == 0 ? 0x8000u : (uint32_t)(128 + tid) << 8);
+        for (uint64_t j = at; j < end; j += 256) {
+            const int n = (int)min((uint64_t)256, end - j);
+            __syncthreads();
+            for (int i = tid; i < n; i += RG_STATES) {
+                const RangeStep s = range_step(A.syms[j + i]);
+                st[i] = make_uint4(s.mu, s.mv, s.keep, s.k);
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (int i = 0; i < n; i++) {
+                const uint4 v = st[i];
+                b = range_next(b, RangeStep{v.x, v.y, v.z, v.w});
+            }
+        }
+        A.rgMap[slot * RG_STATES + tid] = (uint8_t)((b >> 16) & 0x7F);
+    }
+}
+
+// the value each chunk starts with: one warp per tile, the maps staged 32 chunks at a time
+__global__ void __launch_bounds__(32) k_rg_chain(EntArgs A) {
+    __shared__ __align__(16) uint8_t map[2][32][RG_STATES];
+    __shared__ uint8_t first[32];
+    if (A.status->error) return;
+    const uint32_t t = blockIdx.x;
+    const int lane = threadIdx.x;
+    const uint64_t slot0 = rg_slot0(A, t);
+    const uint32_t nc = rg_chunks(A, t);
+    uint32_t cur = 0;
+    uint4 v[8];
+    auto fetch = [&](uint32_t k0) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t q = i * 32 + lane;   // 16 bytes of the 32 x 128
+            if (k0 + q / 8 < nc) v[i] = reinterpret_cast<const uint4 *>(A.rgMap + (slot0 + k0) * RG_STATES)[q];
+        }
+    };
+    fetch(0);
+    for (uint32_t k0 = 0, z = 0; k0 < nc; k0 += 32, z ^= 1) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) reinterpret_cast<uint4 *>(&map[z][0][0])[i * 32 + lane] = v[i];
+        const bool has = k0 + lane < nc && A.rgStart[slot0 + k0 + lane] != ~0ull;
+        const uint32_t live = __ballot_sync(0xffffffffu, has);
+        if (k0 + 32 < nc) fetch(k0 + 32);
+        __syncwarp();
+        if (lane == 0)
+            for (int i = 0; i < 32; i++) {
+                first[i] = (uint8_t)cur;
+                if ((live >> i) & 1) cur = map[z][i][cur];
+            }
+        __syncwarp();
+        cur = __shfl_sync(0xffffffffu, cur, 0);
+        if (k0 + lane < nc) A.rgFirst[slot0 + k0 + lane] = first[lane];
+        __syncwarp();
+    }
+}
+
+// every chunk from its start value, one thread each: the step's term of the code value and its shift (term | shift << 16,
+// in place of the step), and the chunk's bits.  The start value is known to its upper 8 bits here; the low byte, which
+// only the first step's term contains, is what the chunk before ended with (added by k_rg_bits).
+__global__ void __launch_bounds__(32) k_rg_walk(EntArgs A) {
+    if (A.status->error) return;
+    const uint64_t ns = rg_slots(A);
+    for (uint64_t slot = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; slot < ns; slot += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t t, k, bits = 0;
+        const uint64_t at = A.rgStart[slot];
+        if (at != ~0ull) {
+            rg_find(A, slot, t, k);
+            const uint32_t n = (uint32_t)(rg_end(A, slot, t, k) - at);
+            uint32_t *p = A.syms + at;
+            uint32_t b = range_bits(k == 0 ? 0x8000u : (uint32_t)(128 + A.rgFirst[slot]) << 8);
+            uint32_t ahead[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) ahead[i] = i < n ? p[i] : 0u;
+            for (uint32_t j0 = 0; j0 < n; j0 += 8) {
+                uint32_t now[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) now[i] = ahead[i];
+#pragma unroll
+                for (int i = 0; i < 8; i++) ahead[i] = j0 + 8 + i < n ? p[j0 + 8 + i] : 0u;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    if (j0 + i >= n) break;
+                    const uint32_t e = now[i], r = range_of(b);
+                    const uint32_t u = (e & STEP_FIRST) ? r : (((r >> 8) * (e >> 22)) >> 1) + step_ev(e) + 4u;
+                    b = range_next(b, range_step(e));
+                    const uint32_t d = 15u + 127u - (b >> 23);
+                    p[j0 + i] = (r - u) | (d << 16);
+                    bits += d;
+                }
+            }
+            A.rgLast[slot] = (uint8_t)range_of(b);
+        }
+        A.rgBits[slot] = bits;
+    }
+}
+
+// bytes of a tile whose steps shifted c bits out: the whole bytes sent while coding (the first after 9 bits), then the
+// flush, which sends what is left of c + 1 bits
+__device__ __forceinline__ uint32_t rg_bytes(uint64_t c) {
+    const uint64_t n0 = c >= 9 ? (c - 9) / 8 + 1 : 0;
+    const int s = (int)((long long)c - 9 - 8 * (long long)n0) + 10;
+    return (uint32_t)(n0 + (s + 7) / 8);
+}
+// a tile's digits: bit i of the payload (0 the first byte's top bit) is bit i + 16 from the top of the digits; a term of
+// 16 bits after c shifted bits starts at bit c + 15
+__device__ __forceinline__ uint64_t rg_digits(uint32_t bytes) { return (bytes + 1) / 2 + 4; }
+__device__ __forceinline__ uint32_t *rg_digit0(const EntArgs &A, uint32_t t) { return A.rgDigit + A.symBegin[t] + 16 * (uint64_t)t; }
+
+// per tile: the bits before each chunk, the payload's size, the digits cleared
+__global__ void __launch_bounds__(SCAN_T) k_rg_offs(EntArgs A) {
+    __shared__ uint32_t sh[32];
+    if (A.status->error) return;
+    const uint32_t t = blockIdx.x;
+    const uint64_t slot0 = rg_slot0(A, t);
+    const uint32_t nc = rg_chunks(A, t);
+    uint64_t carry = 0;
+    for (uint32_t b = 0; b < nc; b += SCAN_T) {
+        const uint32_t i = b + threadIdx.x;
+        const uint32_t v = i < nc ? A.rgBits[slot0 + i] : 0;
+        uint32_t tot;
+        const uint32_t e = cta_exclusive(v, sh, &tot);
+        if (i < nc) A.rgBit0[slot0 + i] = carry + e;
+        carry += tot;
+        __syncthreads();
+    }
+    const uint32_t bytes = rg_bytes(carry);
+    if (threadIdx.x == 0) {
+        A.tileBytes[t] = bytes;
+        A.tileBits[t] = carry;
+        if (rg_digits(bytes) > A.symBegin[t + 1] - A.symBegin[t] + 16) ent_fail(A, IS_ENT_ERR_OUTPUT);
+    }
+    uint32_t *d = rg_digit0(A, t);
+    const uint64_t nd = min(rg_digits(bytes), A.symBegin[t + 1] - A.symBegin[t] + 16);
+    for (uint64_t i = threadIdx.x; i < nd; i += SCAN_T) d[i] = 0;
+}
+
+// the terms into the digits: one warp per chunk.  A digit's sum stays below 2^32: the terms from a place on add up to
+// less than the range there.
+__global__ void __launch_bounds__(128) k_rg_bits(EntArgs A) {
+    if (A.status->error) return;
+    const uint64_t ns = rg_slots(A);
+    const int lane = threadIdx.x & 31;
+    for (uint64_t slot = (uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5); slot < ns; slot += (uint64_t)gridDim.x * 4) {
+        const uint64_t at = A.rgStart[slot];
+        if (at == ~0ull) continue;
+        uint32_t t, k;
+        rg_find(A, slot, t, k);
+        const uint64_t end = rg_end(A, slot, t, k);
+        uint32_t *dig = rg_digit0(A, t);
+        uint64_t c = A.rgBit0[slot];
+        uint32_t next = at + lane < end ? A.syms[at + lane] : 0u;
+        if (k && lane == 0) {   // the low byte of the range the chunk starts with
+            uint64_t q = slot - 1;
+            while (A.rgStart[q] == ~0ull) q--;   // (a tile's first chunk has a start)
+            next += A.rgLast[q];
+        }
+        for (uint64_t j = at; j < end; j += 32) {
+            const uint32_t w = next, x = w & 0xFFFFu, d = w >> 16;
+            next = j + 32 + lane < end ? A.syms[j + 32 + lane] : 0u;
+            uint32_t inc = d;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            const uint64_t q = c + inc - d + 15;
+            const uint32_t a = (uint32_t)q & 15;
+            // the terms that start in the same digit are neighbours: summed first, then one addition per digit
+            uint32_t hi = x >> a, lo = (x << (16 - a)) & 0xFFFFu;
+            const uint32_t base = (uint32_t)(q >> 4) - (uint32_t)((c + 15) >> 4);
+            const uint32_t same = __match_any_sync(0xffffffffu, base);
+            hi = __reduce_add_sync(same, hi);
+            lo = __reduce_add_sync(same, lo);
+            if (lane == __ffs(same) - 1) {
+                if (hi) atomicAdd(dig + (q >> 4), hi);
+                if (lo) atomicAdd(dig + (q >> 4) + 1, lo);
+            }
+            c += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0 && end == A.symBegin[t + 1]) {   // the flush rounds up by 0x3FFF after the last step
+            const uint64_t q = c + 15;
+            const uint32_t a = (uint32_t)q & 15;
+            atomicAdd(dig + (q >> 4), 0x3FFFu >> a);
+            atomicAdd(dig + (q >> 4) + 1, (0x3FFFu << (16 - a)) & 0xFFFFu);
+        }
+    }
+}
+
+// the carries from a tile's last digit to its first, 1024 digits at a time (each warp's 32 digits by one addition of
+// their generate / propagate bits, then the warps' the same way), the flush's last bit, and the bytes into the payload
+__global__ void __launch_bounds__(SCAN_T) k_rg_carry(EntArgs A) {
+    __shared__ uint32_t gw[32], pw[32], cw;
+    if (A.status->error) return;
+    const uint32_t t = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t bytes = A.tileBytes[t];
+    const uint64_t c = A.tileBits[t], nd = rg_digits(bytes);
+    const uint32_t *d = rg_digit0(A, t);
+    uint8_t *out = A.out + A.tileOff[t];
+    uint32_t cin = 0;
+    for (uint64_t b = 0; b < nd; b += SCAN_T) {
+        const uint64_t i = b + threadIdx.x;            // digits counted from the last
+        uint32_t v = 0;
+        if (i < nd) {
+            const uint64_t m = nd - 1 - i;
+            const uint32_t d0 = d[m], d1 = m + 1 < nd ? d[m + 1] : 0u, d2 = m + 2 < nd ? d[m + 2] : 0u;
+            const uint32_t n0 = (d0 & 0xFFFFu) + (d1 >> 16), n1 = (d1 & 0xFFFFu) + (d2 >> 16);
+            v = (n0 & 0xFFFFu) + (n1 >> 16);
+        }
+        const uint32_t gen = __ballot_sync(0xffffffffu, v > 0xFFFFu), prop = __ballot_sync(0xffffffffu, v == 0xFFFFu);
+        // carries of a + b: a = gen | prop, b = gen; a warp generates without a carry in, propagates with one
+        const uint32_t a = gen | prop;
+        const uint64_t w0 = (uint64_t)a + gen, w1 = w0 + 1;
+        if (lane == 0) { gw[warp] = (uint32_t)(w0 >> 32); pw[warp] = (uint32_t)(w1 >> 32); }
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t G = __ballot_sync(0xffffffffu, gw[lane] != 0), P = __ballot_sync(0xffffffffu, pw[lane] != 0);
+            const uint64_t sum = (uint64_t)P + G + cin;
+            if (lane == 0) cw = (uint32_t)sum ^ P ^ G;   // carry into each warp
+            cin = (uint32_t)(sum >> 32);
+        }
+        __syncthreads();
+        const uint32_t wc = (cw >> warp) & 1;
+        const uint32_t cr = ((uint32_t)(w0 + wc) ^ a ^ gen) >> lane & 1;
+        v = (v + cr) & 0xFFFFu;
+        if (i < nd) {
+            const uint64_t m = nd - 1 - i;
+            if (m > 0) {
+#pragma unroll
+                for (int z = 0; z < 2; z++) {
+                    const uint64_t at = 2 * (m - 1) + z;   // byte of the payload, bits 8 at .. 8 at + 7
+                    uint32_t x = (z ? v : v >> 8) & 0xFFu;
+                    const long long last = (long long)c - 8 * (long long)at;   // the flush sets bit c and clears those after it
+                    if (last < 0) x = 0;
+                    else if (last < 8) x = (x & (0xFF00u >> last)) | (0x80u >> last);
+                    if (at < bytes) out[at] = (uint8_t)x;
+                }
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -822,19 +1263,54 @@ __global__ void __launch_bounds__(SCAN_T) k_ent_offsets(EntArgs A) {
         A.status->bytes = carry;
     }
 }
-__global__ void k_ent_pack(EntArgs A) {
-    const uint32_t g = blockIdx.x;
-    if (A.status->error) return;
-    const uint64_t src = 2 * A.symBegin[g] + 16 * (uint64_t)g, dst = A.tileOff[g];
-    const uint32_t n = A.tileBytes[g];
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) A.out[dst + i] = A.tbytes[src + i];
-}
-
 // ---------------------------------------------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------------------------------------------
+namespace {
+struct CdfList { std::vector<uint16_t> id, off; std::vector<uint8_t> n; };
+template <typename T> void cdf_field(CdfList &L, size_t at) {   // the CDFs of one field of av1g_cdfs: symbols, then the counter
+    constexpr size_t per = std::extent<T, std::rank<T>::value - 1>::value;
+    for (size_t o = 0; o < sizeof(T) / 2; o += per) {
+        const size_t off = at / 2 + o;
+        L.id[off / 3] = (uint16_t)L.off.size();
+        L.off.push_back((uint16_t)off);
+        L.n.push_back((uint8_t)(per - 1));
+    }
+}
+const CdfList &cdf_list() {
+    static const CdfList list = [] {
+        CdfList L;
+        L.id.assign(NCDF / 3 + 1, 0);
+#define IS_CDF_FIELD(f) cdf_field<decltype(av1g_cdfs::f)>(L, offsetof(av1g_cdfs, f));
+        IS_CDF_FIELD(y_mode) IS_CDF_FIELD(uv_mode_cfl_not_allowed) IS_CDF_FIELD(uv_mode_cfl_allowed) IS_CDF_FIELD(angle_delta)
+        IS_CDF_FIELD(partition_w8) IS_CDF_FIELD(partition_w16) IS_CDF_FIELD(partition_w32) IS_CDF_FIELD(partition_w64) IS_CDF_FIELD(skip)
+        IS_CDF_FIELD(intra_tx_set1) IS_CDF_FIELD(intra_tx_set2) IS_CDF_FIELD(cfl_sign) IS_CDF_FIELD(cfl_alpha) IS_CDF_FIELD(txb_skip)
+        IS_CDF_FIELD(eob_pt_16) IS_CDF_FIELD(eob_pt_32) IS_CDF_FIELD(eob_pt_64) IS_CDF_FIELD(eob_pt_128) IS_CDF_FIELD(eob_pt_256)
+        IS_CDF_FIELD(eob_pt_512) IS_CDF_FIELD(eob_pt_1024) IS_CDF_FIELD(eob_extra) IS_CDF_FIELD(dc_sign) IS_CDF_FIELD(coeff_base_eob)
+        IS_CDF_FIELD(coeff_base) IS_CDF_FIELD(coeff_br)
+#undef IS_CDF_FIELD
+        return L;
+    }();
+    return list;
+}
+}  // namespace
+
 cudaError_t ent_upload(const TableBlob &B) {
     cudaError_t e = upload_common(B);
+    const CdfList &L = cdf_list();
+    const int nCdf = (int)L.off.size();
+    if (e == cudaSuccess && nCdf > NID_MAX) e = cudaErrorInvalidValue;
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_cdfId, L.id.data(), L.id.size() * 2);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_cdfOff, L.off.data(), L.off.size() * 2);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_cdfN, L.n.data(), L.n.size());
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_nCdf, &nCdf, sizeof nCdf);
+    std::vector<uint16_t> order;
+    for (int big = 0; big < 2; big++) {
+        for (int i = 0; i < nCdf; i++)
+            if ((L.n[i] > 4) == (big == 1)) order.push_back((uint16_t)i);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_cdfOrder, order.data(), order.size() * 2);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ent_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CsSmem));
     uint8_t w[22], h[22];
     for (int i = 0; i < 22; i++) { w[i] = AV1G_T(Mi_Width_Log2)[i]; h[i] = AV1G_T(Mi_Height_Log2)[i]; }
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_miWLog2, w, sizeof w);
@@ -908,7 +1384,8 @@ struct Plan {
     size_t bytes = 0;
     // offsets in the scratch
     size_t oFr, oBases, oMi, oCtx, oType, oEob, oSbFirst, oTxbBlock, oTxbCnt, oHeadCnt, oHeadW, oPartB, oPartT, oSyms,
-        oBegin, oPre, oTb, oTileBytes, oResult, oOut;
+        oBegin, oRgStart, oRgBit0, oRgBits, oRgFirst, oRgLast, oRgMap, oRgDigit, oTileBits, oCsTab, oCsStart, oCsLen, oTileBytes, oResult, oOut;
+    uint32_t csPitch = 0;
 };
 
 size_t al(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -983,12 +1460,23 @@ int plan(const is_ent_frame *frames, int n, uint64_t cap, Plan &P, std::string *
     P.oPartT = take(4ull * (npT + 1));
     P.oSyms = take(4ull * P.cap);
     P.oBegin = take(8ull * (P.nTiles + 1));
-    const uint64_t preN = 2 * P.cap + 16ull * P.nTiles;
-    P.oPre = take(2 * preN);
-    P.oTb = take(preN);
+    const uint64_t outN = 2 * P.cap + 16ull * P.nTiles;   // at most 15 bits a symbol, and the flush
+    const uint64_t slots = P.cap / RG_CH + P.nTiles + 1;
+    P.oRgStart = take(8 * slots);
+    P.oRgBit0 = take(8 * slots);
+    P.oRgBits = take(4 * slots);
+    P.oRgFirst = take(slots);
+    P.oRgLast = take(slots);
+    P.oRgMap = take((uint64_t)RG_STATES * slots);
+    P.oRgDigit = take(4 * (P.cap + 16ull * P.nTiles));
+    P.oTileBits = take(8ull * P.nTiles);
+    P.csPitch = ((uint32_t)cdf_list().off.size() + 7) & ~7u;
+    P.oCsTab = take(4ull * P.csPitch * (P.cap / CS_B + P.nTiles + 1));
+    P.oCsStart = take(4ull * P.csPitch * P.nTiles);
+    P.oCsLen = take(4ull * P.csPitch * P.nTiles);
     P.oTileBytes = take(4ull * P.nTiles);
     P.oResult = take(sizeof(is_ent_status) + 8ull * (P.nTiles + 1));
-    P.oOut = take(preN);
+    P.oOut = take(outN);
     P.bytes = o;
     return IS_OK;
 }
@@ -1031,8 +1519,18 @@ int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, s
     A.syms = (uint32_t *)(S + P.oSyms);
     A.cap = P.cap;
     A.symBegin = (uint64_t *)(S + P.oBegin);
-    A.pre = (uint16_t *)(S + P.oPre);
-    A.tbytes = S + P.oTb;
+    A.rgStart = (uint64_t *)(S + P.oRgStart);
+    A.rgBit0 = (uint64_t *)(S + P.oRgBit0);
+    A.rgBits = (uint32_t *)(S + P.oRgBits);
+    A.rgFirst = S + P.oRgFirst;
+    A.rgLast = S + P.oRgLast;
+    A.rgMap = S + P.oRgMap;
+    A.rgDigit = (uint32_t *)(S + P.oRgDigit);
+    A.tileBits = (uint64_t *)(S + P.oTileBits);
+    A.csTab = (uint32_t *)(S + P.oCsTab);
+    A.csStart = (uint32_t *)(S + P.oCsStart);
+    A.csLen = (uint32_t *)(S + P.oCsLen);
+    A.csPitch = P.csPitch;
     A.tileBytes = (uint32_t *)(S + P.oTileBytes);
     A.status = (is_ent_status *)(S + P.oResult);
     A.tileOff = (uint64_t *)(S + P.oResult + sizeof(is_ent_status));
@@ -1053,7 +1551,7 @@ int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, s
     if (e == cudaSuccess) {
         k_ent_blocks<<<grid(P.nB, 256), 256, 0, s>>>(A);
         if (P.nT) k_ent_txb<<<grid(P.nT, 128), 128, 0, s>>>(A);
-        k_ent_sb<<<grid(P.nSb, 64), 64, 0, s>>>(A);
+        k_ent_sb<<<grid(P.nSb, SB_WARPS), SB_WARPS * 32, 0, s>>>(A);
         const uint32_t npB = (P.nB + SCAN_T - 1) / SCAN_T, npT = (P.nT + SCAN_T - 1) / SCAN_T;
         uint32_t *partB = (uint32_t *)(S + P.oPartB), *partT = (uint32_t *)(S + P.oPartT);
         k_scan_local<<<npB, SCAN_T, 0, s>>>(A.headCnt, P.nB, partB);
@@ -1067,9 +1565,26 @@ int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, s
         k_ent_tiles<<<grid(P.nTiles, 128), 128, 0, s>>>(A);
         k_ent_emit_head<<<grid(P.nB, 256), 256, 0, s>>>(A);
         if (P.nT) k_ent_emit_txb<<<grid(P.nT, 128), 128, 0, s>>>(A);
-        k_ent_code<<<P.nTiles, 64, 0, s>>>(A);
+        // the batches' and chunks' counts are known on the device only: grids for the symbol capacity, at most a few waves
+        // of the GPU
+        const uint64_t batches = P.cap / CS_B + P.nTiles;
+        const CdfList &L = cdf_list();
+        const int nSmall = (int)std::count_if(L.n.begin(), L.n.end(), [](uint8_t v) { return v <= 4; }), nLarge = (int)L.n.size() - nSmall;
+        const int sw = (nSmall + 7) / 8, wpt = sw + (nLarge + 1) / 2;
+        k_ent_count<<<(unsigned)std::min<uint64_t>(batches, 592), CS_T, 0, s>>>(A);
+        k_ent_place<<<P.nTiles, SCAN_T, 0, s>>>(A);
+        k_ent_scatter<<<(unsigned)std::min<uint64_t>(batches, 296), CS_T, sizeof(CsSmem), s>>>(A);
+        k_ent_adapt<<<(unsigned)wpt * P.nTiles, 32, 0, s>>>(A, sw, nSmall, nLarge, wpt);
+        const uint64_t slots = P.cap / RG_CH + P.nTiles;
+        auto wave = [&](uint64_t perCta, unsigned most) { return (unsigned)std::min<uint64_t>(most, grid(slots, (int)perCta)); };
+        k_rg_starts<<<wave(64, 1184), 64, 0, s>>>(A);
+        k_rg_map<<<wave(1, 2368), RG_STATES, 0, s>>>(A);
+        k_rg_chain<<<P.nTiles, 32, 0, s>>>(A);
+        k_rg_walk<<<wave(32, 2368), 32, 0, s>>>(A);
+        k_rg_offs<<<P.nTiles, SCAN_T, 0, s>>>(A);
         k_ent_offsets<<<1, SCAN_T, 0, s>>>(A);
-        k_ent_pack<<<P.nTiles, 256, 0, s>>>(A);
+        k_rg_bits<<<wave(4, 2368), 128, 0, s>>>(A);
+        k_rg_carry<<<P.nTiles, SCAN_T, 0, s>>>(A);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

@@ -162,6 +162,28 @@ def test_device_entropy_matches_av1core(enc, w, h, q, bd, c444, seed):
     _check(enc, im, w, h, q, bd, c444)
 
 
+def _edge_picture(kind, w, h, bd, c444):
+    """Pictures at the edges of the coder's batches (4096 symbols) and range chunks (1024 steps): flat (long stretches of
+    symbol 0, from which no chunk can start), noise (several batches and chunks per SB, Golomb bits), half (both)."""
+    dt, top = (np.uint16, 1023) if bd == 10 else (np.uint8, 255)
+    rng = np.random.default_rng(w * 1000 + h)
+    out = []
+    for ph, pw in ((h, w),) + (((h, w) if c444 else ((h + 1) // 2, (w + 1) // 2)),) * 2:
+        p = np.full((ph, pw), top // 2, dt)
+        if kind != "flat":
+            x0 = pw // 2 if kind == "half" else 0
+            p[:, x0:] = rng.integers(0, top + 1, (ph, pw - x0))
+        out.append(p)
+    return tuple(out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,w,h,q,bd,c444", [("flat", 8, 8, 120, 8, False), ("flat", 1000, 700, 200, 8, False), ("noise", 64, 64, 1, 8, False),
+                                                ("noise", 200, 136, 2, 10, True), ("half", 330, 250, 8, 8, True), ("half", 4200, 72, 40, 8, False)])
+def test_device_entropy_batch_and_chunk_edges(enc, kind, w, h, q, bd, c444):
+    _check(enc, _edge_picture(kind, w, h, bd, c444), w, h, q, bd, c444)
+
+
 @pytest.mark.gpu
 def test_device_entropy_reference_picture(enc):
     """The reference's CfL test picture at three qindex values."""
