@@ -36,6 +36,7 @@ static __constant__ int c_anShapeStart[AN_SHAPES + 1], c_anShapeStartBig[ANB_GRO
 template <typename Px, int BUFI> struct AnWarp {
     int32_t buf[BUFI];
     int16_t q[1024];
+    uint32_t words[EVAL_WORDS];           // packed levels of the evaluations
     Px pred[BUFI > 2048 ? 4096 : 1024];   // predictions of the tasks' candidates, W x H per group
     int predC[8];                         // candidate whose prediction a group's slice holds (-1: none)
     i64 taskJ[8];
@@ -128,8 +129,8 @@ __device__ __noinline__ void an_block(const FrameDesc &F, const Px *tile, AnWarp
     int nc = nm;
     if (nsl == 0 && bs >= AV1G_BLOCK_8X8) {
         const i64 jd = (lane < nm && is_dir(cand_mode(S.cand[lane]))) ? js : INF;
-        const int l0 = warp_argmin(jd, lane);
-        const int l1 = warp_argmin(lane == l0 ? INF : jd, lane);
+        const int l0 = warp_argmin(jd);
+        const int l1 = warp_argmin(lane == l0 ? INF : jd);
         const int b0 = l0 >= 0 ? cand_mode(S.cand[l0]) : -1, b1 = l1 >= 0 ? cand_mode(S.cand[l1]) : -1;
         const int nd = (b0 >= 0 ? 6 : 0) + (b1 >= 0 ? 6 : 0);   // 12 with the plain form's two directional modes
         __syncwarp();
@@ -148,7 +149,7 @@ __device__ __noinline__ void an_block(const FrameDesc &F, const Px *tile, AnWarp
     const int kMax = nsl > 0 ? F.slRdK : F.rdK;   // a shortlisted block: its best slRdK candidates only
 #pragma unroll
     for (int k = 0; k < K_TOP; k++) {
-        top[k] = warp_argmin(js, lane);
+        top[k] = warp_argmin(js);
         if (top[k] >= 0 && k < kMax) nK = k + 1;
         if (lane == top[k]) js = INF;
     }
@@ -170,8 +171,8 @@ __device__ __noinline__ void an_block(const FrameDesc &F, const Px *tile, AnWarp
         if (S.predC[grp] != c) grp_predict(m, pangle(m, cand_delta(c)), lw, lh, A, L, dcv, tp, g, G);
         __syncwarp();
         if (g == 0) S.predC[grp] = c;
-        const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, T};
-        return grp_eval<BD, Px>(txSz, ResFn<Px>{src, TW, tp, lw, nullptr}, e, tb, tq, g, G);
+        const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, F.dcM, F.acM, T};
+        return grp_eval<BD, TABS_GLOBAL, Px>(txSz, ResFn<Px>{src, TW, tp, lw, nullptr}, e, tb, tq, S.words + grp * eval_words(txSz), g, G);
     };
     i64 bestJ = INF;
     int bestK = 0, bestTx = AV1G_DCT_DCT;
@@ -213,7 +214,7 @@ __device__ __noinline__ void an_block(const FrameDesc &F, const Px *tile, AnWarp
     if (F.txKeep && set != AV1G_TX_SET_DCTONLY) {
         i64 v = lane < 16 ? S.txJ[lane] : INF;
         for (int k = 0; k < F.txKeep; k++) {
-            const int b = warp_argmin(v, lane);
+            const int b = warp_argmin(v);
             if (b < 0) break;
             txMask |= 1u << b;
             if (lane == b) v = INF;

@@ -23,6 +23,7 @@
 #include "is_frame.cuh"
 #include "is_units.cuh"
 #include "is_tiny.cuh"
+#include "is_small.cuh"
 #include "is_dp.cuh"
 #include "is_sched.cuh"
 #include "is_learn.cuh"
@@ -333,6 +334,11 @@ int upload_tables(int dev) {
                     e = cudaErrorInvalidValue;
         }
         if (kDr23 != AV1G_T(Dr_Intra_Derivative)[23] || kDr45 != AV1G_T(Dr_Intra_Derivative)[45] || kDr67 != AV1G_T(Dr_Intra_Derivative)[67]) e = cudaErrorInvalidValue;
+        for (int lw = 2; lw <= 4; lw++)
+            for (int lh = 2; lw + lh <= 6; lh++)
+                for (int t = 0; t < 19; t++)
+                    if (AV1G_T(Tx_Width_Log2)[t] == lw && AV1G_T(Tx_Height_Log2)[t] == lh && AV1G_T(Transform_Row_Shift)[t] != small_row_shift(lw, lh))
+                        e = cudaErrorInvalidValue;
         // the analysis task lists and where each shape's tasks start in them
         B.anTask = an_tasks(0);
         B.anTaskBig = an_tasks(1);
@@ -668,6 +674,8 @@ static int prepare_batch(is_handle *h, const is_frame *fr, int n) {
         lambda_fx(f->qindex, bd, &F.lam, &F.sqlam);
         F.dcQ = AV1G_T(Dc_Qlookup)[g10][f->qindex];
         F.acQ = AV1G_T(Ac_Qlookup)[g10][f->qindex];
+        F.dcM = quant_recip(F.dcQ);
+        F.acM = quant_recip(F.acQ);
         // the image's format group: its ready queue and counters; img indexes the group's descriptors
         F.readyQ = (unsigned long long *)(base + offQG[grp[i]]);
         F.rq = h->bRq + 2 * grp[i];

@@ -146,28 +146,28 @@ __device__ __forceinline__ void smem_poison(unsigned char *base, size_t bytes, i
     for (size_t i = tid; i < bytes / 4; i += nt) reinterpret_cast<uint32_t *>(base)[i] = 0xA5C3E1F7u;
 }
 
+// ---- address spaces: an out-of-line function does not know where its pointers lead and would use generic accesses,
+// which take the global path's latency even when they end in shared memory ----
+#define IS_SHARED_PTR(p) __builtin_assume(__isShared(p))
+#define IS_GLOBAL_PTR(p) __builtin_assume(__isGlobal(p))
+enum TabSpace { TABS_SHARED, TABS_GLOBAL };   // where an evaluation's rate tables are
+
 // ---- warp helpers ----
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
-__device__ __forceinline__ int warp_sum(int v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+__device__ __forceinline__ int warp_sum(int v) { return __reduce_add_sync(0xffffffffu, v); }
+__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
+// the sum of 32-bit lane values in 64 bits (the 16-bit halves apart: no carry is lost)
+__device__ __forceinline__ i64 warp_sum_wide(int v) {
+    return (i64)__reduce_add_sync(0xffffffffu, v >> 16) * 65536 + __reduce_add_sync(0xffffffffu, v & 0xFFFF);
 }
-__device__ __forceinline__ i64 warp_sum64(i64 v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ int warp_max(int v) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-// index of the smallest (v, i) over the warp; the first of equal values (a serial scan's pick); -1 if all are >= INF
-__device__ __forceinline__ int warp_argmin(i64 v, int i) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const i64 ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-        if (ov < v || (ov == v && oi < i)) { v = ov; i = oi; }
-    }
-    return v < INF ? i : -1;
+// the lane of the smallest v >= 0 over the warp, the first of equal values (a serial scan's pick); -1 if all are >= INF
+__device__ __forceinline__ int warp_argmin(i64 v) {
+    const int hi = (int)(v >> 32);
+    const uint32_t lo = (uint32_t)v;
+    const int mh = __reduce_min_sync(0xffffffffu, hi);
+    const uint32_t ml = __reduce_min_sync(0xffffffffu, hi == mh ? lo : 0xFFFFFFFFu);
+    const unsigned best = __ballot_sync(0xffffffffu, hi == mh && lo == ml);
+    return mh < (int)(INF >> 32) ? __ffs(best) - 1 : -1;
 }
 
 // The best (at most 3) tx types of an analysed block by open-loop RD cost, the first evaluated of equal costs ahead:
@@ -419,15 +419,19 @@ __device__ __forceinline__ int hadamard4_sum(int *d) {
 template <typename P, typename O>
 __device__ __noinline__ int pred4_x(int mode, int pAng, int sy, int sx, int lw, int lh, const P *A, const P *L, int dcv, const P *src, int sp,
                                     O *out) {
+    IS_SHARED_PTR(A);
+    IS_SHARED_PTR(L);
     int d[16];
     pred4_inl(mode, pAng, sy, sx, lw, lh, A, L, dcv, d);
     if (out) {
+        IS_SHARED_PTR(out);
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) out[((sy + i) << lw) + sx + j] = (O)d[i * 4 + j];
         return 0;
     }
+    IS_SHARED_PTR(src);
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -444,6 +448,9 @@ __device__ __forceinline__ int pred4_satd(int mode, int pAng, int sy, int sx, in
 // values, the work spread over every lane instead of one lane per sub-block)
 template <typename P, typename O>
 __device__ __noinline__ void grp_predict(int mode, int pAng, int lw, int lh, const P *A, const P *L, int dcv, O *out, int g, int G) {
+    IS_SHARED_PTR(A);
+    IS_SHARED_PTR(L);
+    IS_SHARED_PTR(out);
     const int nsx = 1 << (lw - 2), nsub = 1 << (lw + lh - 4);
     if (nsub < G) {
         for (int q = g; q < (1 << (lw + lh)); q += G) out[q] = (O)pred_px(mode, pAng, q >> lw, q & ((1 << lw) - 1), lw, lh, A, L, dcv);
@@ -495,7 +502,9 @@ template <int BD, typename P>
 __device__ __forceinline__ int warp_dc(const P *A, const P *L, int haveL, int haveA, int lw, int lh) {
     const int w = 1 << lw, h = 1 << lh, lane = lane_id();
     int sa = 0, sl = 0;
+#pragma unroll 2
     for (int k = lane; k < w; k += 32) sa += A[k];
+#pragma unroll 2
     for (int k = lane; k < h; k += 32) sl += L[k];
     sa = warp_sum(sa);
     sl = warp_sum(sl);
@@ -551,7 +560,47 @@ __device__ __forceinline__ void fwd_mem_n(int kind, int32_t *p, int stride, int 
         }
     }
 }
+// the column pass of an evaluation: the residual of one column (src, row stride sp, minus pred, row stride 1 << lw; or,
+// without src, the array arr of that row stride) through the network into p (n <= nout values); returns its energy
+template <int N, typename Px>
+__device__ __forceinline__ i64 fwd_res_n(int kind, const Px *src, int sp, const Px *pred, int lw, const int32_t *arr, int32_t *p, int stride,
+                                         int pre, int nout, int post) {
+    int32_t T[N];
+    i64 en = 0;
+    if (src) {
+#pragma unroll
+        for (int i = 0; i < N; i++) T[i] = (int)src[i * sp] - (int)pred[i << lw];
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) T[i] = arr[i << lw];
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        if (N == 64 || nout < 0) en += (i64)T[i] * T[i];
+        T[i] = T[i] * (1 << pre);
+    }
+    fwd1d<N>(kind, T);
+    const int no = nout < 0 ? -nout : nout;
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (i < no) p[i * stride] = (T[i] + (1 << (post - 1))) >> post;   // (post = log2 of the width: at least 2)
+    return en;
+}
+// nout negative: the energy is wanted (a tx size with a 64-sample side), of |nout| values kept
+template <typename Px>
+__device__ __noinline__ i64 fwd1d_res(int kind, int n, const Px *src, int sp, const Px *pred, int lw, const int32_t *arr, int32_t *p, int stride,
+                                      int pre, int nout, int post) {
+    IS_SHARED_PTR(p);
+    switch (n) {
+    case 4: return fwd_res_n<4, Px>(kind, src, sp, pred, lw, arr, p, stride, pre, nout, post);
+    case 8: return fwd_res_n<8, Px>(kind, src, sp, pred, lw, arr, p, stride, pre, nout, post);
+    case 16: return fwd_res_n<16, Px>(kind, src, sp, pred, lw, arr, p, stride, pre, nout, post);
+    case 32: return fwd_res_n<32, Px>(0, src, sp, pred, lw, arr, p, stride, pre, nout, post);
+    default: return fwd_res_n<64, Px>(0, src, sp, pred, lw, arr, p, stride, pre, nout, post);
+    }
+}
 static __device__ __noinline__ void fwd1d_mem(int kind, int n, int32_t *p, int stride, int pre, int nout, int rect, int post) {
+    IS_SHARED_PTR(p);
     switch (n) {
     case 4: fwd_mem_n<4>(kind, p, stride, pre, nout, rect, post); break;
     case 8: fwd_mem_n<8>(kind, p, stride, pre, nout, rect, post); break;
@@ -600,14 +649,19 @@ struct ResFn {
 
 // ---- lane groups: G lanes (a power of two) evaluate one task; reductions stay inside the aligned group ----
 __device__ __forceinline__ int grp_sum(int v, int G) {
+    if (G == 32) return __reduce_add_sync(0xffffffffu, v);
+#pragma unroll 1
     for (int o = G >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 __device__ __forceinline__ i64 grp_sum64(i64 v, int G) {
+#pragma unroll 1
     for (int o = G >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 __device__ __forceinline__ int grp_max(int v, int G) {
+    if (G == 32) return __reduce_max_sync(0xffffffffu, v);
+#pragma unroll 1
     for (int o = G >> 1; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
@@ -636,6 +690,7 @@ __device__ __forceinline__ int task_buf_ints(int txSz) { return txh(txSz) * (txw
 // ---------------------------------------------------------------------------------------------------------------
 struct EvalIn {
     int txType, plane, skipCtx, dcCtx, intraDir, dcQ, acQ;
+    uint32_t dcM, acM;   // quant_recip of dcQ, acQ
     RateTabs T;          // cost table of the image's q-context, scans, base-context offsets
 };
 struct EvalOut { i64 D, R; int eob; };
@@ -733,62 +788,151 @@ __device__ __forceinline__ int coeff_bits(int c, int eob, const int16_t *q, cons
     return b;
 }
 
-// One evaluation (group of G lanes, all 32 lanes of the warp call it together with the same txSz): residual into
-// buf, forward transform in place (columns, then rows), dead-zone quantisation into q (zbin 21/32, rounding 3/8 of
-// the step, the reference's 0.656 / 0.375; levels capped at 16383), transform-domain distortion, exact rate.  The
-// coefficients stay in buf (th x tw, row stride W + 1).
-template <int BD, typename Px>
+// words of scratch an evaluation packs its levels into: rows of ceil(tw / 8) words of 8 levels (4 bits each) for th + 4
+// rows, capped at 3, then the same capped at 15, then the base contexts' sums; a round of 32 / G tasks (grp_size,
+// round_group) takes at most EVAL_WORDS
+constexpr int EVAL_WORDS = 448;
+__device__ __forceinline__ int eval_words(int txSz) {
+    const int tw = min(txw(txSz), 32), th = min(txh(txSz), 32);
+    return (2 * (th + 4) + th) * ((tw + 7) >> 3);
+}
+
+// One evaluation (group of G lanes, all 32 lanes of the warp call it together with the same txSz): residual and forward
+// transform (columns into buf, then rows in place), dead-zone quantisation into q (zbin 21/32, rounding 3/8 of the step,
+// the reference's 0.656 / 0.375; levels capped at 16383), transform-domain distortion, exact rate.  The coefficients stay
+// in buf (th x tw, row stride W + 1); words: eval_words() words of scratch of the group.
+//
+// A lane takes 8 coefficients of a row at a time, without branches (the lanes' latencies overlap, and a division costs a
+// multiplication by the step's reciprocal), and leaves their levels packed, 4 bits each: the context sums of 8 coefficients
+// are then a few shifts and additions of words.  Before, each coefficient in scan order loaded and bounds-checked its 5
+// neighbours and its ranges' 3: quantisation and rate of a 16x16 block took 24 k cycles of 38 k.
+template <int BD, int TSP, typename Px>
 __device__ __noinline__ EvalOut grp_eval_x(int txSz, const Px *rsrc, int rsp, const Px *rpred, int rlw, const int32_t *rarr, int txType,
-                                           int plane, int skipCtx, int dcCtx, int intraDir, int dcQ, int acQ, const uint16_t *cost,
-                                           const uint16_t *scanT, const uint8_t *baseCtx, int32_t *buf, int16_t *q, int g, int G) {
-    // the arguments come as scalars and the structures are rebuilt here, in registers: a structure passed by address
-    // would live in the caller's local memory and be re-read after every store through buf / q
-    const ResFn<Px> rf{rsrc, rsp, rpred, rlw, rarr};
-    EvalIn e;
-    e.txType = txType; e.plane = plane; e.skipCtx = skipCtx; e.dcCtx = dcCtx; e.intraDir = intraDir; e.dcQ = dcQ; e.acQ = acQ;
-    e.T.cost = cost; e.T.scan = scanT; e.T.baseCtx = baseCtx;
+                                           int plane, int skipCtx, int dcCtx, int intraDir, int dcQ, int acQ, uint32_t dcM, uint32_t acM,
+                                           const uint16_t *cost, const uint16_t *scanT, const uint8_t *baseCtx, int32_t *buf, int16_t *q,
+                                           uint32_t *words, int g, int G) {
+    IS_SHARED_PTR(buf);
+    IS_SHARED_PTR(q);
+    IS_SHARED_PTR(words);
+    if (TSP == TABS_SHARED) { IS_SHARED_PTR(cost); IS_SHARED_PTR(scanT); IS_SHARED_PTR(baseCtx); }
+    else { IS_GLOBAL_PTR(cost); IS_GLOBAL_PTR(scanT); IS_GLOBAL_PTR(baseCtx); }
     const TxRt d = tx_rt(txSz, BD);
-    const int ck = col_kind(e.txType), rk = row_kind(e.txType);
+    const int ck = col_kind(txType), rk = row_kind(txType);
     const bool big = d.W == 64 || d.H == 64;
     i64 en = 0;
-    for (int j = g; j < d.W; j += G) {
-        for (int i = 0; i < d.H; i++) {
-            const int r = rf(i, j);
-            en += r * r;
-            buf[i * d.TS + j] = r;
-        }
-        fwd1d_mem(ck, d.H, buf + j, d.TS, d.s0, d.th, 0, d.s1);
-    }
+#pragma unroll 1
+    for (int j = g; j < d.W; j += G)
+        en += fwd1d_res<Px>(ck, d.H, rarr ? nullptr : rsrc + j, rsp, rarr ? nullptr : rpred + j, rlw, rarr ? rarr + j : nullptr, buf + j, d.TS, d.s0,
+                            big ? -d.th : d.th, d.s1);
     __syncwarp();
+#pragma unroll 1
     for (int i = g; i < d.th; i += G) fwd1d_mem(rk, d.W, buf + i * d.TS, 1, 0, d.tw, d.rect, d.s2);
     __syncwarp();
-    const int den = dq_denom(txSz);
+    const int den = dq_denom(txSz), ltw = d.ltw, lsw = min(ltw, 3), sw = 1 << lsw;   // coefficients per item: 8, or the width if it is 4
+    const int ps = (d.tw + 7) >> 3, nItems = d.n >> lsw;                             // words per packed row
+    uint32_t *p3 = words, *p15 = words + (d.th + 4) * ps, *sums = p15 + (d.th + 4) * ps;
     i64 dist = 0, kept = 0;
-    for (int idx = g; idx < d.n; idx += G) {
-        const int v = buf[(idx >> d.ltw) * d.TS + (idx & (d.tw - 1))];
-        const int step = idx == 0 ? e.dcQ : e.acQ;
-        const int a = abs(v) * den, S = step << FB;
-        int l = 0;
-        if (a * 32 >= 21 * S) l = min((8 * a + 3 * S) / (8 * S), 16383);
-        const int qv = v < 0 ? -l : l;
-        q[idx] = (int16_t)qv;
-        const int dq = l ? dequant<BD>(qv, step, den) * (1 << FB) : 0;
-        const i64 df = (i64)(v - dq);
-        dist += df * df;
-        kept += (i64)v * v;
+#pragma unroll 1
+    for (int k = g; k < 4 * ps; k += G) {   // the rows below
+        p3[d.th * ps + k] = 0;
+        p15[d.th * ps + k] = 0;
+    }
+#pragma unroll 1
+    for (int it = g; it < nItems; it += G) {
+        const int r = it >> (ltw - lsw), s = it & ((1 << (ltw - lsw)) - 1), c0 = s << lsw;
+        const int32_t *v8 = buf + r * d.TS + c0;
+        uint32_t w3 = 0, w15 = 0, lv[4];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int v = j < sw ? v8[j] : 0;
+            const bool dc = j == 0 && it == 0;
+            const int step = dc ? dcQ : acQ, a = abs(v), ad = a * den, St = step << FB;
+            const uint32_t n = (uint32_t)(8 * ad + 3 * St), dv = (uint32_t)(8 * St);
+            uint32_t u = __umulhi(n, dc ? dcM : acM);   // n / dv or one less
+            u += n - u * dv >= dv;
+            const int l = ad * 32 >= 21 * St ? min((int)u, 16383) : 0;
+            const int qv = v < 0 ? -l : l;
+            // |dequantised|: 24 bits, the tx size's denominator, clamped to 2^(7 + BD) below and one less above zero
+            const int dq = min((int)((uint32_t)((l * step) & 0xFFFFFF) >> (den >> 1)), (1 << (7 + BD)) - (v >= 0 ? 1 : 0));
+            const int df = a - dq * (1 << FB);
+            dist += (i64)df * df;
+            kept += (i64)a * a;
+            w3 |= (uint32_t)min(l, 3) << (4 * j);
+            w15 |= (uint32_t)min(l, 15) << (4 * j);
+            if (j & 1) lv[j >> 1] |= (uint32_t)qv << 16; else lv[j >> 1] = (uint32_t)qv & 0xFFFFu;
+        }
+        if (lsw == 3) *reinterpret_cast<uint4 *>(q + (it << 3)) = make_uint4(lv[0], lv[1], lv[2], lv[3]);
+        else *reinterpret_cast<uint2 *>(q + (it << 2)) = make_uint2(lv[0], lv[1]);
+        p3[r * ps + s] = w3;
+        p15[r * ps + s] = w15;
     }
     dist = grp_sum64(dist, G);
     __syncwarp();
-    const uint16_t *scan = get_scan(e.T, txSz, e.txType);
+    const uint16_t *scan = scanT + c_scanOff[txSz][txType == AV1G_IDTX ? 0 : tx_class(txType)];
     int last = 0;
+#pragma unroll 4
     for (int c = g; c < d.n; c += G)
         if (q[scan[c]]) last = c + 1;
     const int eob = grp_max(last, G);
+    const int cls = tx_class(txType), ptype = plane > 0;
+    const int txSzCtx = (ST(Tx_Size_Sqr)[txSz] + ST(Tx_Size_Sqr_Up)[txSz] + 1) >> 1;
+    const uint16_t *cBase = cost + ci_base(txSzCtx, ptype, 0), *cBr = cost + ci_br(min(txSzCtx, (int)AV1G_TX_32X32), ptype, 0);
+    const uint16_t *cEob = cost + ci_base_eob(txSzCtx, ptype, 0);
     int b = 0;
-    const int cls = tx_class(e.txType);
-    for (int c = g; c < eob; c += G) b += coeff_bits(c, eob, q, scan, txSz, cls, e.plane > 0, e.dcCtx, e.T);
+    // per 8 coefficients: the base contexts' sums, the signs, and the ranges of the levels above 2
+    if (eob) {
+#pragma unroll 1
+        for (int it = g; it < nItems; it += G) {
+            const int r = it >> (ltw - lsw), s = it & ((1 << (ltw - lsw)) - 1);
+            const bool last = s == ps - 1;
+            auto right = [&](const uint32_t *p, int k) -> uint32_t { return __funnelshift_r(p[0], last ? 0u : p[1], 4 * k); };   // from k columns on
+            const uint32_t *a = p3 + r * ps + s, *x = p15 + r * ps + s;
+            uint32_t m = right(a, 1) + a[ps];
+            if (cls == AV1G_TX_CLASS_2D) m += right(a + ps, 1) + right(a, 2) + a[2 * ps];
+            else if (cls == AV1G_TX_CLASS_HORIZ) m += right(a, 2) + right(a, 3) + right(a, 4);
+            else m += a[2 * ps] + a[3 * ps] + a[4 * ps];
+            sums[r * ps + s] = m;
+            const uint32_t w = x[0];
+            uint32_t nz = w | w >> 1;
+            nz = (nz | nz >> 2) & 0x11111111u;
+            b += 256 * __popc(nz);
+            if (!nz) continue;
+            const uint32_t xr = right(x, 1), xd = x[ps];
+            const uint32_t xc = cls == AV1G_TX_CLASS_2D ? right(x + ps, 1) : cls == AV1G_TX_CLASS_HORIZ ? right(x, 2) : x[2 * ps];
+            const uint32_t w3 = a[0];
+            uint32_t bg = (w3 & w3 >> 1) & 0x11111111u;   // levels above 2
+#pragma unroll 1
+            for (; bg; bg &= bg - 1) {
+                const int sh = __ffs((int)bg) - 1, j = (s << lsw) + (sh >> 2), l = (int)(w >> sh) & 15;
+                const int mg = min(((int)(xr >> sh & 15) + (int)(xd >> sh & 15) + (int)(xc >> sh & 15) + 1) >> 1, 6);
+                const int near = cls == AV1G_TX_CLASS_2D ? (r < 2 && j < 2) : cls == AV1G_TX_CLASS_HORIZ ? j == 0 : r == 0;
+                const uint16_t *cr = cBr + ((r | j) == 0 ? mg : near ? mg + 7 : mg + 14) * IS_CD(coeff_br, 3);
+                const int rem = l - 3, full = (rem * 11) >> 5;   // rem / 3: at most 4 symbols
+                b += full * cr[3];
+                if (full < 4) b += cr[rem - 3 * full];
+                if (l == 15) {
+                    const int v = abs((int)q[(r << ltw) + j]);
+                    if (v > 14) b += (2 * (31 - __clz(v - 14)) + 1) * 256;
+                }
+            }
+        }
+        if (g == 0 && q[0]) b += cost[ci_dc_sign(ptype, dcCtx) + (q[0] < 0)] - 256;   // the DC sign has its own contexts
+    }
+    __syncwarp();
+    // the base symbols in scan order
+    const int off0 = ST(Coeff_Base_Pos_Ctx_Offset)[0], off1 = ST(Coeff_Base_Pos_Ctx_Offset)[1], off2 = ST(Coeff_Base_Pos_Ctx_Offset)[2];
+#pragma unroll 4
+    for (int c = g; c < eob; c += G) {
+        const int pos = scan[c], r = pos >> ltw, col = pos & (d.tw - 1), sh = (col & 7) * 4, at = r * ps + (col >> 3);
+        const int l3 = (int)(p3[at] >> sh) & 3, mag = (int)(sums[at] >> sh) & 15;
+        int ctx = min((mag + 1) >> 1, 4);
+        if (cls == AV1G_TX_CLASS_2D) ctx = pos == 0 ? 0 : ctx + baseCtx[txSz * 25 + min(r, 4) * 5 + min(col, 4)];
+        else { const int k = cls == AV1G_TX_CLASS_VERT ? r : col; ctx += k == 0 ? off0 : k == 1 ? off1 : off2; }
+        const int ectx = c == 0 ? 0 : c <= d.n / 8 ? 1 : c <= d.n / 4 ? 2 : 3;
+        b += *(c == eob - 1 ? cEob + ectx * IS_CD(coeff_base_eob, 3) + l3 - 1 : cBase + ctx * IS_CD(coeff_base, 3) + l3);
+    }
     EvalOut o;
-    o.R = grp_sum(b, G) + base_bits(txSz, e.txType, e.plane, e.skipCtx, e.intraDir, e.T.cost, eob);
+    o.R = grp_sum(b, G) + base_bits(txSz, txType, plane, skipCtx, intraDir, cost, eob);
     o.D = dist << d.dsh;
     if (big) {
         en = grp_sum64(en, G);
@@ -799,10 +943,10 @@ __device__ __noinline__ EvalOut grp_eval_x(int txSz, const Px *rsrc, int rsp, co
     o.eob = eob;
     return o;
 }
-template <int BD, typename Px>
-__device__ __forceinline__ EvalOut grp_eval(int txSz, const ResFn<Px> &rf, const EvalIn &e, int32_t *buf, int16_t *q, int g, int G) {
-    return grp_eval_x<BD, Px>(txSz, rf.src, rf.sp, rf.pred, rf.lw, rf.arr, e.txType, e.plane, e.skipCtx, e.dcCtx, e.intraDir, e.dcQ, e.acQ,
-                              e.T.cost, e.T.scan, e.T.baseCtx, buf, q, g, G);
+template <int BD, int TSP, typename Px>
+__device__ __forceinline__ EvalOut grp_eval(int txSz, const ResFn<Px> &rf, const EvalIn &e, int32_t *buf, int16_t *q, uint32_t *words, int g, int G) {
+    return grp_eval_x<BD, TSP, Px>(txSz, rf.src, rf.sp, rf.pred, rf.lw, rf.arr, e.txType, e.plane, e.skipCtx, e.dcCtx, e.intraDir, e.dcQ, e.acQ,
+                                   e.dcM, e.acM, e.T.cost, e.T.scan, e.T.baseCtx, buf, q, words, g, G);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -869,6 +1013,7 @@ __device__ __forceinline__ uint32_t inv_mem_n(int kind, int32_t *p, int stride, 
     return e;
 }
 static __device__ __noinline__ uint32_t inv1d_mem(int kind, int n, int32_t *p, int stride, int r, int preRect, int post, int clampBits) {
+    IS_SHARED_PTR(p);
     switch (n) {
     case 4: return inv_mem_n<4>(kind, p, stride, r, preRect, post, clampBits);
     case 8: return inv_mem_n<8>(kind, p, stride, r, preRect, post, clampBits);
@@ -883,6 +1028,7 @@ static __device__ __noinline__ uint32_t inv1d_mem(int kind, int n, int32_t *p, i
 // clamp to colClampRange, column transforms, Round2(., 4)); returns the OR of the conformance flags (group)
 template <int BD>
 __device__ __noinline__ uint32_t grp_inverse(int txSz, const int16_t *q, int txType, int dcQ, int acQ, int32_t *buf, int g, int G) {
+    IS_SHARED_PTR(buf);
     const TxRt d = tx_rt(txSz, BD);
     constexpr int rowR = BD + 8, colR = (BD + 6) > 16 ? BD + 6 : 16;
     const int den = dq_denom(txSz);

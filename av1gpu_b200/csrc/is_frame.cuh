@@ -60,6 +60,7 @@ struct __align__(16) FrameDesc {
     int shNbx[22], shNby[22];
     long long lam, sqlam;                     // lambda, sqrt(lambda) in 1/256
     int dcQ, acQ;
+    uint32_t dcM, acM;                        // quant_recip of dcQ, acQ
     Leaf *leaves;                             // [nSb * 256]
     uint16_t *nLeaves;                        // [nSb]
     av1g_block *oBlocks;                      // [nSb * 256]
@@ -103,6 +104,12 @@ struct __align__(16) FrameDesc {
     int waitIters;
     int poison;                               // fill shared memory with a pattern at kernel start (is_set_poison)
 };
+
+// a quantiser step's divisions by 64 step as multiplications: (n M) >> 32 is n / (64 step) or one less (n < 2^32)
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint32_t quant_recip(int step) { return 0xFFFFFFFFu / (64u * (unsigned)step); }
 
 // error codes written to FrameDesc::err by the kernels
 constexpr int KERR_WAIT_LEAF = 2;    // a leaf dependency wait of the closed loop ran out of its iteration budget

@@ -19,16 +19,16 @@
 #pragma once
 #include "is_dev.cuh"
 #include "is_frame.cuh"
+#include "is_small.cuh"
 
 namespace is {
 
 // warps per CTA: independent workers, as many as the shared memory of one CTA per SM holds (at most 8; rc_warps below)
 constexpr int RC_MAX_WARPS = 8;
-// per-warp scratch: a task round of tx sizes up to 32 x 32 (32 / G tasks of H x (W + 1) int32: at most 16 x 80 in the
-// small sizes' single round (G >= 2, 4x16), 4 x 272 / 2 x 544 / 1 x 1056 in the others (round_group's G)) and
-// predictions up to 32 x 32 (16 x 64 in the single round); the luma of a leaf with a 64-sample side (rare: large flat
-// blocks) uses the CTA's one large buffer (RcBig) instead, under a lock
-constexpr int RC_BUF_INTS = 1280;
+// per-warp scratch: a task round of tx sizes up to 32 x 32 (32 / G tasks of H x (W + 1) int32: at most 4 x 272, 2 x 544 or
+// 1 x 1056 by round_group's G; the small sizes' packed rows take 16 x 41 words) and predictions up to 32 x 32; the luma of
+// a leaf with a 64-sample side (rare: large flat blocks) uses the CTA's one large buffer (RcBig) instead, under a lock
+constexpr int RC_BUF_INTS = 1088;
 // bounded waits (defaults; FrameDesc::waitIters / readyWaitNs carry the values of a run): a wait that runs out records
 // an error and moves on, and once any error is recorded no further wait starts (the host discards the result)
 constexpr int LEAF_WAIT_ITERS = 1 << 20;
@@ -38,6 +38,7 @@ constexpr int LEAF_WAIT_ITERS = 1 << 20;
 constexpr int TRACE_STAMPS = 10;
 constexpr long long READY_WAIT_NS = 4000000000ll;
 
+static_assert(EVAL_WORDS * 4 <= 1024 * 2, "packed levels in one of RcWarp::qb");
 template <typename Px, int SS> struct RcWarp {   // SS: chroma subsampling (1 4:2:0, 0 4:4:4)
     int32_t buf[RC_BUF_INTS];  // evaluation scratch (32 / G tasks) and the inverse transform's residual (tx <= 32 x 32)
     int16_t q[1024];           // levels of the tasks of a round
@@ -69,6 +70,7 @@ template <typename Px, int SS, int NW> struct RcSmem {
     RateStage T;                         // scans, base-context offsets (and the cost table of q-context 0)
     RcBig<Px> big;
     uint16_t cost[3][NCDF];              // the cost tables of q-contexts 1 .. 3 (the images of a batch mix qindex)
+    SmallTabs small;                     // tables of the small sizes' evaluation
     RcSlot<Px, SS> ws[NW];
 };
 template <typename Px, int SS> constexpr size_t rc_smem_bytes(int warps) {
@@ -146,21 +148,26 @@ __device__ __forceinline__ void rec_edges(const P *plane, int pitch, int x, int 
 
 // exact inverse + reconstruction of a tx block (warp), the levels halved until conformant (AV1G_ENC_FIX_RANGE's
 // repair, the reference's cta_inverse_add, k_recon.cuh:140-197); writes prediction + residual into the plane
+// (not inlined, as rc_record and rc_edges_rec: one copy serves every tx block of a leaf)
 template <int BD, typename Px>
-__device__ void rc_reconstruct(int txSz, int txType, int16_t *q, int dcQ, int acQ, const Px *pred, Px *dst, int pitch, int32_t *buf) {
+__device__ __noinline__ void rc_reconstruct(int txSz, int txType, int16_t *q, int dcQ, int acQ, const Px *pred, Px *dst, int pitch, int32_t *buf) {
+    IS_SHARED_PTR(q); IS_SHARED_PTR(pred); IS_SHARED_PTR(buf); IS_GLOBAL_PTR(dst);
     const int lane = lane_id();
     const int W = txw(txSz), H = txh(txSz), n = min(W, 32) * min(H, 32), TS = W + 1;
     bool any = false;
     for (;;) {
         int nz = 0;
+#pragma unroll 2
         for (int i = lane; i < n; i += 32) nz |= q[i] != 0;
         if (!__any_sync(0xffffffffu, nz)) { any = false; break; }
         const uint32_t err = grp_inverse<BD>(txSz, q, txType, dcQ, acQ, buf, lane, 32);
         if (!err) { any = true; break; }
+#pragma unroll 1
         for (int i = lane; i < n; i += 32) q[i] = (int16_t)(q[i] / 2);
         __syncwarp();
     }
     const int lw = 31 - __clz(W);
+#pragma unroll 2
     for (int p = lane; p < W * H; p += 32) {
         const int i = p >> lw, j = p & (W - 1);
         int v = (int)pred[p] + (any ? buf[i * TS + j] : 0);
@@ -206,29 +213,34 @@ __device__ void rc_edges_rec(const FrameDesc &F, int pl, int px, int py, int W, 
 }
 
 // record a finished tx block: eob, culLevel / dc category into the context maps, the txb entry and its levels
-static __device__ int rc_record(const FrameDesc &F, const RateTabs &T, int sb, int plane, int txSz, int txType, int x4, int y4, const int16_t *q,
+static __device__ __noinline__ int rc_record(const FrameDesc &F, const RateTabs &T, int sb, int plane, int txSz, int txType, int x4, int y4, const int16_t *q,
                          int txbIdx, int coefOff) {
+    IS_SHARED_PTR(&F); IS_SHARED_PTR(q);
     const int lane = lane_id();
     const int W = txw(txSz), H = txh(txSz), n = min(W, 32) * min(H, 32);
     const uint16_t *scan = get_scan(T, txSz, txType);
     int last = 0;
+#pragma unroll 2
     for (int c = lane; c < n; c += 32) if (q[scan[c]]) last = c + 1;
     const int eob = warp_max(last);
     int cul = 0;
+#pragma unroll 1
     for (int c = lane; c < eob; c += 32) cul += abs((int)q[scan[c]]);
     cul = min(warp_sum(cul), 63);
     const int dcCat = q[0] < 0 ? 1 : q[0] > 0 ? 2 : 0;
     const int ss = plane ? F.ssx : 0;
     const int stride = F.MiCols >> ss, rows = F.MiRows >> ss;
-    const int w4 = W >> 2, h4 = H >> 2;
+    const int w4 = W >> 2, h4 = H >> 2, lw4 = 31 - __clz(w4);
+#pragma unroll 1
     for (int k = lane; k < w4 * h4; k += 32) {
-        const int yy = y4 + k / w4, xx = x4 + k % w4;
+        const int yy = y4 + (k >> lw4), xx = x4 + (k & (w4 - 1));
         if (yy < rows && xx < stride) {
             F.cLvl[plane][(size_t)yy * stride + xx] = (uint8_t)(eob ? cul : 0);
             F.cDc[plane][(size_t)yy * stride + xx] = (uint8_t)(eob ? dcCat : 0);
         }
     }
     int16_t *oc = F.oCoeffs + (size_t)sb * SB_MAX_COEF + coefOff;
+#pragma unroll 2
     for (int i = lane; i < n; i += 32) oc[i] = q[i];
     if (lane == 0) {
         av1g_txb t;
@@ -292,15 +304,18 @@ __device__ __forceinline__ void rc_txb_ctx(const FrameDesc &F, int plane, int tx
 // a block of H rows of W bytes (<= 64; a W x H <= 32 x 32 block of samples) at src (row pitch in bytes) into dst (row
 // stride W bytes), vector loads of up to 16 bytes (rows and the block's first byte are aligned to its width).  Coherent
 // L2 loads, not the read-only path: a serving session's loop runs while new images are written into reused memory.
-__device__ __forceinline__ void stage_block(const uint8_t *src, int pitch, int W, int H, uint8_t *dst) {
+static __device__ __noinline__ void stage_block(const uint8_t *src, int pitch, int W, int H, uint8_t *dst) {
     const int lane = lane_id();
     if (W >= 16) {
-        const int v = W >> 4;
-        for (int k = lane; k < v * H; k += 32)
-            reinterpret_cast<uint4 *>(dst)[k] = __ldcg(reinterpret_cast<const uint4 *>(src + (size_t)(k / v) * pitch) + (k % v));
+        const int lv = 27 - __clz(W);   // log2 of the row's 16-byte words
+#pragma unroll 2
+        for (int k = lane; k < (H << lv); k += 32)
+            reinterpret_cast<uint4 *>(dst)[k] = __ldcg(reinterpret_cast<const uint4 *>(src + (size_t)(k >> lv) * pitch) + (k & ((1 << lv) - 1)));
     } else if (W == 8) {
+#pragma unroll 1
         for (int k = lane; k < H; k += 32) reinterpret_cast<uint2 *>(dst)[k] = __ldcg(reinterpret_cast<const uint2 *>(src + (size_t)k * pitch));
     } else {
+#pragma unroll 1
         for (int k = lane; k < H; k += 32) reinterpret_cast<uint32_t *>(dst)[k] = __ldcg(reinterpret_cast<const uint32_t *>(src + (size_t)k * pitch));
     }
 }
@@ -332,8 +347,9 @@ __device__ __forceinline__ int unit_leaf(const FrameDesc &F, int sb, int li, int
 static __device__ __noinline__ bool rc_wait(const FrameDesc &F, int sb, int li, int sbr, int sbc, int rTop, int c0, int c1, int cLeft, int r0,
                                      int r1, int st, int level, int tC0, int tC1, int tR0) {
     const int lane = lane_id();
-    const int nTop = c1 > c0 ? (c1 - c0 + st - 1) / st : 0, nLeft = r1 > r0 ? (r1 - r0 + st - 1) / st : 0;
+    const int nTop = c1 > c0 ? (c1 - c0 + st - 1) >> (st - 1) : 0, nLeft = r1 > r0 ? (r1 - r0 + st - 1) >> (st - 1) : 0;   // (st is 1 or 2)
     bool ok = true;
+#pragma unroll 1
     for (int u = lane; u < nTop + nLeft; u += 32) {
         const int yy = u < nTop ? rTop : r0 + (u - nTop) * st, xx = u < nTop ? c0 + u * st : cLeft;
         const int id = unit_leaf(F, sb, li, sbr, sbc, yy, xx, tC0, tC1, tR0);
@@ -373,7 +389,9 @@ __device__ __forceinline__ bool rc_big_lock(const FrameDesc &F, int &lock) {
 // tile box (mi units) of the 4x4 unit (mi_row, mi_col)
 __device__ __forceinline__ void tile_box(const FrameDesc &F, int mi_row, int mi_col, int &tC0, int &tC1, int &tR0, int &tR1) {
     int tc = 0, tr = 0;
+#pragma unroll 1
     while (tc + 1 < F.tileCols && mi_col >= F.tileColStart[tc + 1]) tc++;
+#pragma unroll 1
     while (tr + 1 < F.tileRows && mi_row >= F.tileRowStart[tr + 1]) tr++;
     tC0 = F.tileColStart[tc]; tC1 = F.tileColStart[tc + 1]; tR0 = F.tileRowStart[tr]; tR1 = F.tileRowStart[tr + 1];
 }
@@ -435,10 +453,10 @@ __device__ __noinline__ int rc_chroma_more(const FrameDesc &F, RcWarp<Px, 0> &Wp
         __threadfence_block();   // the context maps of this leaf's earlier tx blocks (written by this warp)
         int sc, dcc;
         rc_txb_ctx(F, pl, txSz, cx4 + (ox >> 2), cy4 + (oy >> 2), bsize, tC0, tR0, &sc, &dcc);
-        const EvalIn e{uvType, pl, sc, dcc, 0, F.dcQ, F.acQ, T};
+        const EvalIn e{uvType, pl, sc, dcc, 0, F.dcQ, F.acQ, F.dcM, F.acM, T};
         const Px *so = (const Px *)F.src[pl] + (size_t)(cy + oy) * F.spitch[pl] + cx + ox;
         int16_t *lv = Wp.qb[pl - 1];
-        grp_eval<BD, Px>(txSz, ResFn<Px>{so, F.spitch[pl], Wp.pred, lw, nullptr}, e, Wp.buf, lv, lane, 32);
+        grp_eval<BD, TABS_SHARED, Px>(txSz, ResFn<Px>{so, F.spitch[pl], Wp.pred, lw, nullptr}, e, Wp.buf, lv, reinterpret_cast<uint32_t *>(Wp.qb[2 - pl]), lane, 32);
         Px *dst = (Px *)F.rec[pl] + (size_t)(cy + oy) * F.rpitch[pl] + cx + ox;
         rc_reconstruct<BD, Px>(txSz, uvType, lv, F.dcQ, F.acQ, Wp.pred, dst, F.rpitch[pl], Wp.buf);
         eobs |= rc_record(F, T, sb, pl, txSz, uvType, cx4 + (ox >> 2), cy4 + (oy >> 2), lv, txb0 + *tIdx, coef0 + *tIdx * nq);
@@ -448,7 +466,7 @@ __device__ __noinline__ int rc_chroma_more(const FrameDesc &F, RcWarp<Px, 0> &Wp
 }
 
 template <int BD, typename Px, int SS>
-__device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, const RateTabs &T, int sb, int li, unsigned long long *trace) {
+__device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, const RateTabs &T, const SmallTabs *ST6, int sb, int li, unsigned long long *trace) {
     const int lane = lane_id();
     const Leaf lf = F.leaves[(size_t)sb * SB_MAX_LEAVES + li];
     const int bsize = lf.bsize;
@@ -552,120 +570,125 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
         int32_t *lbuf = bigTx ? Big.buf : Wp.buf;
         Px *lpred = bigTx ? Big.pred : Wp.pred;
         int16_t *best = Wp.qb[0];
+        uint32_t *words = reinterpret_cast<uint32_t *>(Wp.qb[1]);   // the evaluations' packed levels
         i64 bestJ = INF;
         int bestC = br.cand[0], bestT = br.tx;
         bool have = false;
-        int curG = 0;
-        // tasks (candidate, tx type) in rounds of 32 / G (G per pass: round_group); costs compared in task order (first
-        // of equal costs wins); the round's winner, if it beats the best so far, leaves its levels in `best`
-        auto run = [&](const int *tcand, const int *ttype, int n) {
-            const int G = round_group(txSz, n), ng = 32 / G, grp = lane / G, g = lane & (G - 1);
-            int32_t *tb = lbuf + grp * task_buf_ints(txSz);
-            int16_t *tq = Wp.q + grp * nq;
-            Px *tp = lpred + grp * (W * H);
-            if (G != curG) {   // the groups' cached predictions belong to another grouping
-                if (lane < 8) Wp.predC[lane] = -1;
-                __syncwarp();
-                curG = G;
-            }
-            for (int r0 = 0; r0 < n; r0 += ng) {
-                const int k = min(r0 + grp, n - 1);
-                const int c = tcand[k], t = ttype[k], m = cand_mode(c);
-                if (Wp.predC[grp] != c) grp_predict(m, pangle(m, cand_delta(c)), lw, lh, A, L, dcv, tp, g, G);
-                __syncwarp();
-                if (g == 0) Wp.predC[grp] = c;
-                const EvalIn e{t, 0, skipCtx, dcCtx, m, F.dcQ, F.acQ, T};
-                const EvalOut o = grp_eval<BD, Px>(txSz, ResFn<Px>{src, srcPitch, tp, lw, nullptr}, e, tb, tq, g, G);
-                if (g == 0 && r0 + grp < n) Wp.taskJ[grp] = o.D + F.lam * (o.R + mbits(c));
-                __syncwarp();
-                int win = -1;
-                for (int u = 0; u < ng && r0 + u < n; u++)
-                    if (Wp.taskJ[u] < bestJ) { bestJ = Wp.taskJ[u]; bestC = tcand[r0 + u]; bestT = ttype[r0 + u]; win = u; have = true; }
-                if (win >= 0)
-                    for (int i = lane; i < nq; i += 32) best[i] = Wp.q[win * nq + i];
-                __syncwarp();
-            }
-        };
         const int nc = max(1, min((int)br.ncand, K_RECHECK));
         // the types pass 2 may try for cand[0]: its open-loop shortlist (with DCT_DCT and the analysis' type), or all
         const uint32_t txAllow = br.txMask ? (uint32_t)br.txMask | (1u << AV1G_DCT_DCT) | (1u << br.tx) : 0xFFFFu;
-        int tcand[8], ttype[8], n1 = 0;
-        for (int k = 0; k < nc; k++) { tcand[n1] = br.cand[k]; ttype[n1] = AV1G_DCT_DCT; n1++; }
-        if (br.tx != AV1G_DCT_DCT) { tcand[n1] = br.cand[0]; ttype[n1] = br.tx; n1++; }
+        const int n1 = nc + (br.tx != AV1G_DCT_DCT);   // pass 1: the first nc candidates with DCT_DCT, the first with its type
         const bool skip1 = n1 == 1;
         if (trace && lane == 0) trace[2] = gtimer();
-        if (W * H <= 64 && set != AV1G_TX_SET_DCTONLY) {
+        const bool small = W * H <= 64;   // (every one of these sizes has the types of TX_SET_INTRA_1)
+        if (small) {
             // Small tx sizes (4x4 .. 8x8, 4x16, 16x4; nine leaves in ten): pass 1 and the pass-2 tx types of BOTH possible
             // pass-1 winners in one round of at most 16 tasks (2 lanes each), then the winner taken in the order of the two
             // passes - pass 1 in task order, then pass 2 of the pass-1 winner in type order, the first of equal costs -
             // which is exactly the result of running pass 2 after pass 1.  A round's latency hardly depends on its task
-            // count, so this saves the second round.
+            // count, so this saves the second round.  Tasks in Wp.cand: candidate (0 / 1) << 4 | type.
             const int c0 = br.cand[0], c1 = nc >= 2 ? br.cand[1] : br.cand[0];
             const int tt = lane & 15;   // pass-2 types: lanes 0-15 for the first candidate, 16-31 for the second
             const bool ok = lane < 16 ? tx_in_set(set, tt) && ((txAllow >> tt) & 1) && !(!skip1 && (tt == AV1G_DCT_DCT || tt == br.tx))
                                       : nc >= 2 && tx_in_set(set, tt) && tt != AV1G_DCT_DCT;
-            const unsigned bal = __ballot_sync(0xffffffffu, ok), m0 = bal & 0xFFFFu, m1 = bal >> 16;
-            const int p1 = skip1 ? 0 : n1, n2a = __popc(m0), n2b = __popc(m1), nt = p1 + n2a + n2b;
-            const int G = nt > 8 ? 2 : nt > 4 ? 4 : 8, grp = lane / G, g = lane & (G - 1);
-            {   // every lane takes part (the evaluation's warp-wide reductions); groups past the last task repeat it
-                const int k = min(grp, nt - 1);
-                int c, ty;
-                if (k < p1) { c = k < nc ? (int)br.cand[k] : c0; ty = k < nc ? AV1G_DCT_DCT : br.tx; }
-                else if (k < p1 + n2a) { c = c0; ty = __fns(m0, 0, k - p1 + 1); }
-                else { c = c1; ty = __fns(m1, 0, k - p1 - n2a + 1); }
-                const int m = cand_mode(c);
-                Px *tp = lpred + grp * (W * H);
-                grp_predict(m, pangle(m, cand_delta(c)), lw, lh, A, L, dcv, tp, g, G);
-                __syncwarp();
-                const EvalIn e{ty, 0, skipCtx, dcCtx, m, F.dcQ, F.acQ, T};
-                const EvalOut o = grp_eval<BD, Px>(txSz, ResFn<Px>{src, srcPitch, tp, lw, nullptr}, e, lbuf + grp * task_buf_ints(txSz),
-                                                   Wp.q + grp * nq, g, G);
-                if (g == 0 && grp < nt) Wp.taskJ[grp] = o.D + F.lam * (o.R + mbits(c));
+            const unsigned bal = __ballot_sync(0xffffffffu, ok);
+            const int p1 = skip1 ? 0 : n1, n2a = __popc(bal & 0xFFFFu), nt = p1 + __popc(bal);
+            if (ok) Wp.cand[p1 + __popc(bal & ((1u << lane) - 1))] = lane;
+            if (lane < p1) Wp.cand[lane] = lane < nc ? lane << 4 | AV1G_DCT_DCT : br.tx;
+            {   // the two candidates' predictions, half a warp each
+                const int c = lane < 16 ? c0 : c1, m = cand_mode(c);
+                grp_predict(m, pangle(m, cand_delta(c)), lw, lh, A, L, dcv, lpred + (lane & 16 ? W * H : 0), lane & 15, 16);
             }
             __syncwarp();
+            {   // every lane takes part (the evaluation's shuffles); pairs past the last task repeat it
+                const int k = lane >> 1, task = Wp.cand[min(k, nt - 1)], c = task & 16 ? c1 : c0;
+                const EvalOut o = small_eval_size<BD, Px>(txSz, src, lpred + (task & 16 ? W * H : 0), task & 15, 0, skipCtx, dcCtx, cand_mode(c), F.dcQ,
+                                                          F.acQ, F.dcM, F.acM, C, ST6, lbuf, reinterpret_cast<uint32_t *>(Wp.qb[0]), Wp.q, k, lane & 1);
+                if (!(lane & 1)) Wp.taskJ[k] = o.D + F.lam * (o.R + mbits(c));
+            }
+            __syncwarp();
+            const i64 j = Wp.taskJ[lane & 15];
             int win = -1;
+            bool first = true;
             if (!skip1) {
-                for (int k = 0; k < p1; k++)
-                    if (Wp.taskJ[k] < bestJ) { bestJ = Wp.taskJ[k]; bestC = k < nc ? (int)br.cand[k] : c0; bestT = k < nc ? AV1G_DCT_DCT : br.tx; win = k; }
-            } else {
-                bestC = c0; bestT = AV1G_DCT_DCT;
+                win = warp_argmin(lane < p1 ? j : INF);
+                first = !(Wp.cand[win] & 16);
             }
-            const bool first = bestC == c0;
-            const int base = first ? p1 : p1 + n2a, cnt = first ? n2a : n2b;
-            const unsigned mk = first ? m0 : m1;
-            for (int j = 0; j < cnt; j++)
-                if (Wp.taskJ[base + j] < bestJ) { bestJ = Wp.taskJ[base + j]; bestT = __fns(mk, 0, j + 1); win = base + j; }
-            if (win >= 0) {
-                have = true;
-                for (int i = lane; i < nq; i += 32) best[i] = Wp.q[win * nq + i];
-            }
-            __syncwarp();
+            const int base = first ? p1 : p1 + n2a, end = first ? p1 + n2a : nt;
+            const int w2 = warp_argmin(lane >= base && lane < end ? j : INF);
+            if (w2 >= 0 && (win < 0 || Wp.taskJ[w2] < Wp.taskJ[win])) win = w2;
+            const int task = Wp.cand[win];
+            bestC = task & 16 ? c1 : c0;
+            bestT = task & 15;
+            best = Wp.q + win * nq;
+            lpred += task & 16 ? W * H : 0;
             if (trace && lane == 0) trace[3] = trace[4] = gtimer();
         } else {
-        if (!skip1) run(tcand, ttype, n1);
-        else { bestC = br.cand[0]; bestT = AV1G_DCT_DCT; }
-        if (trace && lane == 0) trace[3] = gtimer();
-        if (set != AV1G_TX_SET_DCTONLY) {
-            const int c1 = bestC;
-            const bool isC0 = c1 == br.cand[0];
-            int n2 = 0;
-            for (int t = 0; t < 16; t++) {
-                if (!tx_in_set(set, t)) continue;
-                if (!skip1 && (t == AV1G_DCT_DCT || (isC0 && t == br.tx))) continue;
-                if (isC0 && !((txAllow >> t) & 1)) continue;
-                tcand[n2] = c1; ttype[n2] = t; n2++;
+            // tasks (candidate, tx type) in rounds of 32 / G (G per pass: round_group); costs compared in task order (first
+            // of equal costs wins); the round's winner, if it beats the best so far, leaves its levels in `best`.  Both
+            // passes go through one copy of the loop; their tasks lie in Wp.cand (candidate << 4 | type).
+            if (skip1) { bestC = br.cand[0]; bestT = AV1G_DCT_DCT; }
+            int curG = 0;
+#pragma unroll 1
+            for (int pass = skip1 ? 1 : 0; pass < (set != AV1G_TX_SET_DCTONLY ? 2 : 1); pass++) {
+                int n;
+                if (pass == 0) {
+                    n = n1;
+                    if (lane < n) Wp.cand[lane] = lane < nc ? (int)br.cand[lane & 1] << 4 | AV1G_DCT_DCT : (int)br.cand[0] << 4 | br.tx;
+                } else {
+                    const bool isC0 = bestC == br.cand[0];
+                    const int t = lane & 15;
+                    const bool ok = lane < 16 && tx_in_set(set, t) && !(!skip1 && (t == AV1G_DCT_DCT || (isC0 && t == br.tx))) &&
+                                    !(isC0 && !((txAllow >> t) & 1));
+                    const unsigned m = __ballot_sync(0xffffffffu, ok);
+                    n = __popc(m);
+                    if (ok) Wp.cand[__popc(m & ((1u << lane) - 1))] = bestC << 4 | t;
+                }
+                __syncwarp();
+                const int G = round_group(txSz, n), ng = 32 / G, grp = lane / G, g = lane & (G - 1);
+                int32_t *tb = lbuf + grp * task_buf_ints(txSz);
+                int16_t *tq = Wp.q + grp * nq;
+                Px *tp = lpred + grp * (W * H);
+                if (G != curG) {   // the groups' cached predictions belong to another grouping
+                    if (lane < 8) Wp.predC[lane] = -1;
+                    __syncwarp();
+                    curG = G;
+                }
+#pragma unroll 1
+                for (int r0 = 0; r0 < n; r0 += ng) {
+                    const int task = Wp.cand[min(r0 + grp, n - 1)], c = task >> 4, m = cand_mode(c);
+                    if (Wp.predC[grp] != c) grp_predict(m, pangle(m, cand_delta(c)), lw, lh, A, L, dcv, tp, g, G);
+                    __syncwarp();
+                    if (g == 0) Wp.predC[grp] = c;
+                    const EvalIn e{task & 15, 0, skipCtx, dcCtx, m, F.dcQ, F.acQ, F.dcM, F.acM, T};
+                    const EvalOut o = grp_eval<BD, TABS_SHARED, Px>(txSz, ResFn<Px>{src, srcPitch, tp, lw, nullptr}, e, tb, tq, words + grp * eval_words(txSz), g, G);
+                    if (g == 0 && r0 + grp < n) Wp.taskJ[grp] = o.D + F.lam * (o.R + mbits(c));
+                    __syncwarp();
+                    int win = -1;
+#pragma unroll 1
+                    for (int u = 0; u < ng && r0 + u < n; u++)
+                        if (Wp.taskJ[u] < bestJ) { bestJ = Wp.taskJ[u]; win = u; }
+                    if (win >= 0) {
+                        have = true;
+                        bestC = Wp.cand[r0 + win] >> 4;
+                        bestT = Wp.cand[r0 + win] & 15;
+#pragma unroll 1
+                        for (int i = lane; i < nq; i += 32) best[i] = Wp.q[win * nq + i];
+                    }
+                    __syncwarp();
+                }
+                if (trace && lane == 0) trace[3 + pass] = gtimer();
             }
-            run(tcand, ttype, n2);
-        }
-        if (trace && lane == 0) trace[4] = gtimer();
         }
         // the winner's prediction (whole warp) for its levels (single-candidate case) and the reconstruction
         const int bm = cand_mode(bestC);
-        grp_predict(bm, pangle(bm, cand_delta(bestC)), lw, lh, A, L, dcv, lpred, lane, 32);
-        __syncwarp();
-        if (!have) {
-            const EvalIn e{bestT, 0, skipCtx, dcCtx, bm, F.dcQ, F.acQ, T};
-            grp_eval<BD, Px>(txSz, ResFn<Px>{src, srcPitch, lpred, lw, nullptr}, e, lbuf, best, lane, 32);
+        if (!small) {
+            grp_predict(bm, pangle(bm, cand_delta(bestC)), lw, lh, A, L, dcv, lpred, lane, 32);
+            __syncwarp();
+        }
+        if (!small && !have) {
+            const EvalIn e{bestT, 0, skipCtx, dcCtx, bm, F.dcQ, F.acQ, F.dcM, F.acM, T};
+            grp_eval<BD, TABS_SHARED, Px>(txSz, ResFn<Px>{src, srcPitch, lpred, lw, nullptr}, e, lbuf, best, words, lane, 32);
         }
         Px *dst = (Px *)F.rec[0] + (size_t)y * F.rpitch[0] + x;
         rc_reconstruct<BD, Px>(txSz, bestT, best, F.dcQ, F.acQ, lpred, dst, F.rpitch[0], lbuf);
@@ -679,8 +702,10 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
         eobY = rc_record(F, T, sb, 0, txSz, bestT, x >> 2, y >> 2, best, txbBase, coefBase);
         yMode = bm;
         yDelta = cand_delta(bestC);
+        const int lbw = 31 - __clz(bw);
+#pragma unroll 1
         for (int k = lane; k < bw * bh; k += 32) {
-            const int r = mi_row + k / bw, c = mi_col + k % bw;
+            const int r = mi_row + (k >> lbw), c = mi_col + (k & (bw - 1));
             if (r < F.MiRows && c < F.MiCols) F.mYMode[(size_t)r * F.MiCols + c] = (uint8_t)yMode;
         }
     }
@@ -693,6 +718,7 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
     {   // the dependents whose last luma dependency this was enter the ready queue (the taker of a leaf acquires each of
         // its dependencies' flags itself before it reads their data; push_ready releases what this thread wrote)
         __syncwarp();
+#pragma unroll 1
         for (int k = lane; k < relN; k += 32) {
             const uint32_t d = F.revList[relOff + k];
             if (atomicSub(F.depCnt + d, 1) == 1) push_ready(F, d);
@@ -734,16 +760,17 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
         }
         const CtxLd cl1 = rc_txb_ctx_load(F, 1, txSz, cx4, cy4, tC0, tR0), cl2 = rc_txb_ctx_load(F, 2, txSz, cx4, cy4, tC0, tR0);
         const int haveAR = decoded(ss, csr - 1, csc + (W >> 2)), haveBL = decoded(ss, csr + (H >> 2), csc - 1);
+#pragma unroll 1
         for (int q = 1; q <= 2; q++)
             stage_block((const uint8_t *)((const Px *)F.src[q] + (size_t)cy * F.spitch[q] + cx), F.spitch[q] * (int)sizeof(Px), W * (int)sizeof(Px), H,
                         (uint8_t *)Wp.srcS[q]);
         // ---- the edges of U and V (rec_edges' rule on the raw samples) ----
-        Px *A[3], *L[3];
-        int dcv[3];
+        auto eA = [&](int pl) -> Px * { return Wp.ea[pl] + EDGE_OFF; };
+        auto eL = [&](int pl) -> Px * { return Wp.el[pl] + EDGE_OFF; };
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             const int pl = 1 + q;
-            A[pl] = Wp.ea[pl] + EDGE_OFF; L[pl] = Wp.el[pl] + EDGE_OFF;
+            Px *A = eA(pl), *L = eL(pl);
             const Px aW = (Px)__shfl_sync(0xffffffffu, (int)(W > 32 ? ra[q][1] : ra[q][0]), (W - 1) & 31);
             const Px lH = (Px)__shfl_sync(0xffffffffu, (int)(H > 32 ? rl[q][1] : rl[q][0]), (H - 1) & 31);
             const Px a0 = (Px)__shfl_sync(0xffffffffu, (int)ra[q][0], 0), l0 = (Px)__shfl_sync(0xffffffffu, (int)rl[q][0], 0);
@@ -751,20 +778,18 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
             for (int k = 0; k < 2; k++) {
                 const int i = lane + 32 * k;
                 if (i < n) {
-                    A[pl][i] = availUC ? ((!haveAR && i >= W) ? aW : ra[q][k]) : (availLC ? l0 : (Px)((1 << (BD - 1)) - 1));
-                    L[pl][i] = availLC ? ((!haveBL && i >= H) ? lH : rl[q][k]) : (availUC ? a0 : (Px)((1 << (BD - 1)) + 1));
+                    A[i] = availUC ? ((!haveAR && i >= W) ? aW : ra[q][k]) : (availLC ? l0 : (Px)((1 << (BD - 1)) - 1));
+                    L[i] = availLC ? ((!haveBL && i >= H) ? lH : rl[q][k]) : (availUC ? a0 : (Px)((1 << (BD - 1)) + 1));
                 }
             }
             if (lane == 0) {
                 const Px c = (availUC && availLC) ? rcorner[q] : availUC ? a0 : availLC ? l0 : (Px)(1 << (BD - 1));
-                A[pl][-1] = c;
-                L[pl][-1] = c;
+                A[-1] = c;
+                L[-1] = c;
             }
         }
         __syncwarp();
-        for (int pl = 1; pl <= 2; pl++) dcv[pl] = warp_dc<BD>(A[pl], L[pl], availLC, availUC, lw, lh);
-        // the staged sources (row stride W)
-        const Px *sP[3] = {nullptr, (const Px *)Wp.srcS[1], (const Px *)Wp.srcS[2]};
+        const int dcU = warp_dc<BD>(eA(1), eL(1), availLC, availUC, lw, lh), dcV = warp_dc<BD>(eA(2), eL(2), availLC, availUC, lw, lh);
         const bool cflAllowed = bw <= 8 && bh <= 8;
         auto uvbits = [&](int m) -> int { return cflAllowed ? C[ci_uv_cfl(yMode) + m] : C[ci_uv_nocfl(yMode) + m]; };
         auto uvcbits = [&](int c) -> int {
@@ -774,12 +799,13 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
             return b;
         };
         // ---- CfL (spec 7.11.5 luma values; least-squares alpha, then the best of alpha - 1 .. + 1 by SSE) ----
-        int alpha[3] = {0, 0, 0}, cflAvg = 0;
+        int alphaU = 0, alphaV = 0, cflAvg = 0;
         if (cflAllowed) {
             const int maxLumaW = x + 4 * bw, maxLumaH = y + 4 * bh;   // tx_depth 0: one luma tx block, starting inside
             const Px *luma = (const Px *)F.rec[0];
             const int lp = F.rpitch[0];
             int sum = 0;
+#pragma unroll 1
             for (int p = lane; p < W * H; p += 32) {
                 const int i = p >> lw, j = p & (W - 1);
                 int v;
@@ -796,128 +822,149 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
             sum = warp_sum(sum);
             cflAvg = (sum + (1 << (lw + lh - 1))) >> (lw + lh);
             __syncwarp();
-            i64 num1 = 0, num2 = 0, den = 0;
+            // (a lane has at most 32 samples, |l| <= 8184 and |s - dc| <= 1023: its sums fit 32 bits)
+            int num1 = 0, num2 = 0, den1 = 0;
+#pragma unroll 1
             for (int p = lane; p < W * H; p += 32) {
-                const int i = p >> lw, j = p & (W - 1);
-                const i64 l = Wp.cfl[p] - cflAvg;
-                num1 += l * ((int)sP[1][i * W + j] - dcv[1]);
-                num2 += l * ((int)sP[2][i * W + j] - dcv[2]);
-                den += l * l;
+                const int l = Wp.cfl[p] - cflAvg;
+                num1 += l * ((int)Wp.srcS[1][p] - dcU);
+                num2 += l * ((int)Wp.srcS[2][p] - dcV);
+                den1 += l * l;
             }
-            num1 = warp_sum64(num1); num2 = warp_sum64(num2); den = warp_sum64(den);
+            const i64 den = warp_sum_wide(den1);
+#pragma unroll 1
             for (int pl = 1; pl <= 2; pl++) {
-                const i64 num = pl == 1 ? num1 : num2;
-                int a = 0;
-                if (den > 0) {
-                    const i64 n = 64 * num;
-                    a = (int)(n >= 0 ? (2 * n + den) / (2 * den) : -((-2 * n + den) / (2 * den)));
-                }
-                a = max(-16, min(16, a));
-                i64 sse[3] = {0, 0, 0};
+                const int dc = pl == 1 ? dcU : dcV;
+                const i64 n = 64 * warp_sum_wide(pl == 1 ? num1 : num2), na = n >= 0 ? n : -n;
+                // |a| = min(round(|n| / den), 16): the number of k in 1 .. 16 with 2 |n| + den >= 2 k den
+                const int c = __popc(__ballot_sync(0xffffffffu, lane < 16 && den > 0 && 2 * na + den >= 2 * den * (lane + 1)));
+                const int a = n >= 0 ? c : -c;
+                int sse[3] = {0, 0, 0};
+#pragma unroll 1
                 for (int p = lane; p < W * H; p += 32) {
-                    const int i = p >> lw, j = p & (W - 1);
-                    const int l = Wp.cfl[p] - cflAvg, s = sP[pl][i * W + j];
+                    const int l = Wp.cfl[p] - cflAvg, s = Wp.srcS[pl][p];
 #pragma unroll
                     for (int k = 0; k < 3; k++) {
                         const int ak = max(-16, min(16, a + k - 1));
                         const int v = ak * l, sc = v >= 0 ? (v + 32) >> 6 : -((-v + 32) >> 6);
-                        const int pr = min(max(dcv[pl] + sc, 0), (1 << BD) - 1);
-                        sse[k] += (i64)(s - pr) * (s - pr);
+                        const int pr = min(max(dc + sc, 0), (1 << BD) - 1);
+                        sse[k] += (s - pr) * (s - pr);
                     }
                 }
-                for (int k = 0; k < 3; k++) sse[k] = warp_sum64(sse[k]);
-                int bk = 1;
-                for (int k = 0; k < 3; k++) if (sse[k] < sse[bk]) bk = k;
-                alpha[pl] = max(-16, min(16, a + bk - 1));
+#pragma unroll
+                for (int k = 0; k < 3; k++) sse[k] = warp_sum(sse[k]);
+                const int bk = sse[0] < sse[1] ? (sse[2] < sse[0] ? 2 : 0) : sse[2] < sse[1] ? 2 : 1;
+                const int al = max(-16, min(16, a + bk - 1));
+                if (pl == 1) alphaU = al; else alphaV = al;
             }
         }
         // ---- SATD screening of the UV modes over U and V ----
-        const int nsx = W >> 2, nsub2 = 2 * (W >> 2) * (H >> 2);   // items per candidate: U then V 4x4 sub-blocks
-        auto screen = [&](int c0, int c1) {
-            const int items = (c1 - c0) * nsub2;
+        const int lnsx = lw - 2, nsub2 = 2 << (lw + lh - 4), lnsub2 = lw + lh - 3;   // items per candidate: U then V 4x4 sub-blocks
+        Wp.satd[lane] = 0;
+        Wp.cand[lane] = lane < 13 ? cand_pack(lane, 0) : 0;
+        i64 js = INF;
+        // the 13 modes, then (8x8 and larger) +-1..3 around the best directional one: one copy of the loop
+#pragma unroll 1
+        for (int c0 = 0, c1 = 13;;) {
+            __syncwarp();
+            const int items = (c1 - c0) << lnsub2;
+#pragma unroll 1
             for (int it0 = 0; it0 < items; it0 += 32) {
                 const int it = it0 + lane;
-                const int ci = c0 + it / nsub2;
+                const int ci = c0 + (it >> lnsub2);
                 int t = 0;
                 if (it < items) {
-                    const int r = it % nsub2, pl = 1 + (r >= (nsub2 >> 1)), sbk = r % (nsub2 >> 1);
-                    const int sx = (sbk % nsx) * 4, sy = (sbk / nsx) * 4;
+                    const int r = it & (nsub2 - 1), pl = 1 + (r >> (lnsub2 - 1)), sbk = r & ((nsub2 >> 1) - 1);
+                    const int sx = (sbk & ((1 << lnsx) - 1)) * 4, sy = (sbk >> lnsx) * 4;
                     const int c = Wp.cand[ci], m = cand_mode(c);
-                    t = pred4_satd(m, pangle(m, cand_delta(c)), sy, sx, lw, lh, A[pl], L[pl], dcv[pl], sP[pl], W);
+                    t = pred4_satd<Px>(m, pangle(m, cand_delta(c)), sy, sx, lw, lh, eA(pl), eL(pl), pl == 1 ? dcU : dcV, Wp.srcS[pl], W);
                 }
-                for (int o = 16; o > 0; o >>= 1)
-                    if (o < nsub2) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll 1
+                for (int o = min(16, nsub2 >> 1); o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
                 if (it < items && (lane & (nsub2 - 1)) == 0) Wp.satd[ci] += t;
                 __syncwarp();
             }
-        };
-        Wp.satd[lane] = 0;
-        Wp.cand[lane] = lane < 13 ? cand_pack(lane, 0) : 0;
-        __syncwarp();
-        screen(0, 13);
-        i64 js = lane < 13 ? ((i64)Wp.satd[lane] << 14) + F.sqlam * uvcbits(Wp.cand[lane]) : INF;
-        if (bsize >= AV1G_BLOCK_8X8) {
-            const int bm = warp_argmin((lane >= AV1G_V_PRED && lane <= AV1G_D67_PRED) ? js : INF, lane);
+            if (lane >= c0 && lane < c1) js = ((i64)Wp.satd[lane] << 14) + F.sqlam * uvcbits(Wp.cand[lane]);
+            if (c0 || bsize < AV1G_BLOCK_8X8) break;
+            const int bm = warp_argmin((lane >= AV1G_V_PRED && lane <= AV1G_D67_PRED) ? js : INF);
             if (lane < 6) Wp.cand[13 + lane] = cand_pack(bm, lane < 3 ? -(lane + 1) : (lane - 2));
-            __syncwarp();
-            screen(13, 19);
-            if (lane >= 13 && lane < 19) js = ((i64)Wp.satd[lane] << 14) + F.sqlam * uvcbits(Wp.cand[lane]);
+            c0 = 13;
+            c1 = 19;
         }
-        int chosen[UV_K + 1], nch = 0;
+        // the best UV_K modes, then CfL (255) when it has a non-zero alpha
+        int *chosen = Wp.cand + 24;
+        int nch = 0;
+#pragma unroll 1
         for (int k = 0; k < UV_K; k++) {
-            const int b = warp_argmin(js, lane);
+            const int b = warp_argmin(js);
             if (b < 0) break;
-            chosen[nch++] = Wp.cand[b];
+            if (lane == 0) chosen[nch] = Wp.cand[b];
+            nch++;
             if (lane == b) js = INF;
         }
-        if (cflAllowed && (alpha[1] || alpha[2])) chosen[nch++] = 255;
-        int skipCtx[3], dcCtx[3];
-        rc_txb_ctx_finish(F, cl1, 1, txSz, bsize, &skipCtx[1], &dcCtx[1]);
-        rc_txb_ctx_finish(F, cl2, 2, txSz, bsize, &skipCtx[2], &dcCtx[2]);
+        if (cflAllowed && (alphaU || alphaV)) {
+            if (lane == 0) chosen[nch] = 255;
+            nch++;
+        }
+        __syncwarp();
+        int skipU, skipV, dcCtxU, dcCtxV;
+        rc_txb_ctx_finish(F, cl1, 1, txSz, bsize, &skipU, &dcCtxU);
+        rc_txb_ctx_finish(F, cl2, 2, txSz, bsize, &skipV, &dcCtxV);
         // prediction of (plane, candidate) by a group of G lanes into out
         auto predict = [&](int pl, int c, Px *out, int g, int G) {
-            if (c == 255) grp_predict_cfl(lw, lh, dcv[pl], Wp.cfl, alpha[pl], cflAvg, (1 << BD) - 1, out, g, G);
-            else grp_predict(cand_mode(c), pangle(cand_mode(c), cand_delta(c)), lw, lh, A[pl], L[pl], dcv[pl], out, g, G);
+            const int dc = pl == 1 ? dcU : dcV;
+            if (c == 255) grp_predict_cfl(lw, lh, dc, Wp.cfl, pl == 1 ? alphaU : alphaV, cflAvg, (1 << BD) - 1, out, g, G);
+            else grp_predict<Px, Px>(cand_mode(c), pangle(cand_mode(c), cand_delta(c)), lw, lh, eA(pl), eL(pl), dc, out, g, G);
         };
-        // (candidate, plane) tasks in rounds of 32 / G; each candidate's cost = U + V + lambda * its mode bits; the
-        // winner's two planes are evaluated once more for their levels
+        // (candidate, plane) tasks in rounds of 32 / G; each candidate's cost = U + V + lambda * its mode bits; then the
+        // winner's two planes once more for their levels, each a round of one task over the whole warp
         const int nq = min(W, 32) * min(H, 32);
-        i64 pj[2 * (UV_K + 1)];
         const int ntask = 2 * nch;
-        const int G = round_group(txSz, ntask), ng = 32 / G, grp = lane / G, g = lane & (G - 1);
-        int32_t *tb = Wp.buf + grp * task_buf_ints(txSz);
-        int16_t *tq = Wp.q + grp * nq;
-        Px *tp = Wp.pred + grp * (W * H);
-        for (int r0 = 0; r0 < ntask; r0 += ng) {
-            const int k = min(r0 + grp, ntask - 1), c = chosen[k >> 1], pl = 1 + (k & 1);
-            predict(pl, c, tp, g, G);
-            __syncwarp();
-            const int txType = chroma_tx_type(txSz, c == 255 ? AV1G_UV_CFL_PRED : cand_mode(c));
-            const EvalIn e{txType, pl, skipCtx[pl], dcCtx[pl], 0, F.dcQ, F.acQ, T};
-            const EvalOut o = grp_eval<BD, Px>(txSz, ResFn<Px>{sP[pl], W, tp, lw, nullptr}, e, tb, tq, g, G);
-            if (g == 0 && r0 + grp < ntask) Wp.taskJ[grp] = o.D + F.lam * o.R;
-            __syncwarp();
-            for (int u = 0; u < ng && r0 + u < ntask; u++) pj[r0 + u] = Wp.taskJ[u];
-            __syncwarp();
-        }
-        i64 bJ = INF;
-        int bestC = cand_pack(AV1G_DC_PRED, 0);
-        for (int k = 0; k < nch; k++) {
-            const int c = chosen[k];
-            i64 J = pj[2 * k] + pj[2 * k + 1];
+        i64 jc = INF;
+        if (lane < nch) {   // the candidates' mode bits, one lane each
+            const int c = chosen[lane];
             int b;
             if (c == 255) {
-                const int a1 = alpha[1], a2 = alpha[2];
-                const int sU = a1 == 0 ? 0 : a1 < 0 ? 1 : 2, sV = a2 == 0 ? 0 : a2 < 0 ? 1 : 2;
+                const int sU = alphaU == 0 ? 0 : alphaU < 0 ? 1 : 2, sV = alphaV == 0 ? 0 : alphaV < 0 ? 1 : 2;
                 b = uvbits(AV1G_UV_CFL_PRED) + C[ci_cfl_sign() + sU * 3 + sV - 1];
-                if (sU) b += C[ci_cfl_alpha((sU - 1) * 3 + sV) + abs(a1) - 1];
-                if (sV) b += C[ci_cfl_alpha((sV - 1) * 3 + sU) + abs(a2) - 1];
+                if (sU) b += C[ci_cfl_alpha((sU - 1) * 3 + sV) + abs(alphaU) - 1];
+                if (sV) b += C[ci_cfl_alpha((sV - 1) * 3 + sU) + abs(alphaV) - 1];
             } else {
                 b = uvcbits(c);
             }
-            J += F.lam * b;
-            if (J < bJ) { bJ = J; bestC = c; }
+            jc = F.lam * b;
         }
+        const bool small = W * H <= 64;
+        if (small) {
+            // all tasks (at most 6) in one round: the predictions one after the other over the whole warp, two lanes a task
+            // for the evaluation; the winner's levels stay in its tasks' slices
+#pragma unroll 1
+            for (int k = 0; k < ntask; k++) predict(1 + (k & 1), chosen[k >> 1], Wp.pred + k * (W * H), lane, 32);
+            __syncwarp();
+            const int k = lane >> 1, kk = min(k, ntask - 1), c = chosen[kk >> 1], pl = 1 + (kk & 1);
+            const int txType = chroma_tx_type(txSz, c == 255 ? AV1G_UV_CFL_PRED : cand_mode(c));
+            const EvalOut o = small_eval_size<BD, Px>(txSz, Wp.srcS[pl], Wp.pred + kk * (W * H), txType, pl, pl == 1 ? skipU : skipV,
+                                                      pl == 1 ? dcCtxU : dcCtxV, 0, F.dcQ, F.acQ, F.dcM, F.acM, C, ST6, Wp.buf, reinterpret_cast<uint32_t *>(Wp.qb[0]), Wp.q, k, lane & 1);
+            if (!(lane & 1)) Wp.taskJ[k] = o.D + F.lam * o.R;
+            __syncwarp();
+        } else {
+            const int G = round_group(txSz, ntask), ng = 32 / G, grp = lane / G, g = lane & (G - 1);
+            Px *tp = Wp.pred + grp * (W * H);
+#pragma unroll 1
+            for (int r0 = 0; r0 < ntask; r0 += ng) {
+                const int k = min(r0 + grp, ntask - 1), c = chosen[k >> 1], pl = 1 + (k & 1);
+                predict(pl, c, tp, g, G);
+                __syncwarp();
+                const int txType = chroma_tx_type(txSz, c == 255 ? AV1G_UV_CFL_PRED : cand_mode(c));
+                const EvalIn e{txType, pl, pl == 1 ? skipU : skipV, pl == 1 ? dcCtxU : dcCtxV, 0, F.dcQ, F.acQ, F.dcM, F.acM, T};
+                const EvalOut o = grp_eval<BD, TABS_SHARED, Px>(txSz, ResFn<Px>{Wp.srcS[pl], W, tp, lw, nullptr}, e, Wp.buf + grp * task_buf_ints(txSz), Wp.q + grp * nq,
+                                                               reinterpret_cast<uint32_t *>(Wp.qb[0]) + grp * eval_words(txSz), g, G);
+                if (g == 0 && r0 + grp < ntask) Wp.taskJ[r0 + grp] = o.D + F.lam * o.R;
+                __syncwarp();
+            }
+        }
+        if (lane < nch) jc += Wp.taskJ[2 * lane] + Wp.taskJ[2 * lane + 1];
+        const int bc = warp_argmin(jc), bestC = bc >= 0 ? chosen[bc] : cand_pack(AV1G_DC_PRED, 0);
         if (trace && lane == 0) trace[7] = gtimer();
         const bool cfl = bestC == 255;
         uv = cfl ? AV1G_UV_CFL_PRED : cand_mode(bestC);
@@ -929,14 +976,20 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
         const int yt = ST(Max_Tx_Size_Rect)[bsize];
         const int lumaN = min(txw(yt), 32) * min(txh(yt), 32);
         int tIdx = 0;   // coded chroma tx blocks so far
+#pragma unroll 1
         for (int pl = 1; pl <= 2; pl++) {
             Px *dst = (Px *)F.rec[pl] + (size_t)cy * F.rpitch[pl] + cx;
-            int16_t *lv = Wp.qb[pl - 1];
-            predict(pl, bestC, Wp.pred, lane, 32);
-            __syncwarp();
-            const EvalIn e{uvType, pl, skipCtx[pl], dcCtx[pl], 0, F.dcQ, F.acQ, T};
-            grp_eval<BD, Px>(txSz, ResFn<Px>{sP[pl], W, Wp.pred, lw, nullptr}, e, Wp.buf, lv, lane, 32);
-            rc_reconstruct<BD, Px>(txSz, uvType, lv, F.dcQ, F.acQ, Wp.pred, dst, F.rpitch[pl], Wp.buf);
+            const bool kept = small && bc >= 0;   // a small block's winner: its prediction and levels are in its task's slice
+            const int slice = kept ? 2 * bc + pl - 1 : 0;
+            int16_t *lv = kept ? Wp.q + slice * nq : Wp.qb[pl - 1];
+            const Px *pr = Wp.pred + slice * (W * H);
+            if (!kept) {
+                predict(pl, bestC, Wp.pred, lane, 32);
+                __syncwarp();
+                const EvalIn e{uvType, pl, pl == 1 ? skipU : skipV, pl == 1 ? dcCtxU : dcCtxV, 0, F.dcQ, F.acQ, F.dcM, F.acM, T};
+                grp_eval<BD, TABS_SHARED, Px>(txSz, ResFn<Px>{Wp.srcS[pl], W, Wp.pred, lw, nullptr}, e, Wp.buf, lv, reinterpret_cast<uint32_t *>(Wp.qb[2 - pl]), lane, 32);
+            }
+            rc_reconstruct<BD, Px>(txSz, uvType, lv, F.dcQ, F.acQ, pr, dst, F.rpitch[pl], Wp.buf);
             int e2 = rc_record(F, T, sb, pl, txSz, uvType, cx4, cy4, lv, txbBase + 1 + tIdx, coefBase + lumaN + tIdx * nq);
             tIdx++;
             if constexpr (SS == 0) {
@@ -949,8 +1002,8 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
             if (pl == 1) eobU = e2; else eobV = e2;
         }
         duv = cfl ? 0 : cand_delta(bestC);
-        aU = cfl ? alpha[1] : 0;
-        aV = cfl ? alpha[2] : 0;
+        aU = cfl ? alphaU : 0;
+        aV = cfl ? alphaV : 0;
     }
     if (lane == 0) {
         av1g_block b;
@@ -1022,6 +1075,8 @@ __global__ void __launch_bounds__(rc_warps_of<BD, SS>() * 32, 1) k_recon(const F
         }
     }
     if (threadIdx.x == 0) S.big.lock = 0;
+    __syncthreads();
+    small_tabs_stage(S.small, RateTabs{S.T.cost, S.T.scan, S.T.baseCtx}, threadIdx.x, blockDim.x);
     __syncthreads();
     if (warp >= ctl.warps) return;   // (uniform per warp; no CTA barrier follows)
     int *rq = ctl.rq;
@@ -1097,7 +1152,7 @@ __global__ void __launch_bounds__(rc_warps_of<BD, SS>() * 32, 1) k_recon(const F
         }
         const RateTabs T{F.qctx == 0 ? S.T.cost : S.cost[F.qctx - 1], S.T.scan, S.T.baseCtx};
         unsigned long long *trace = traceBase ? traceBase + (size_t)h * TRACE_STAMPS : nullptr;
-        rc_leaf<BD, Px, SS>(F, Wp, S.big, T, (int)(id >> 8), (int)(id & 255), trace);
+        rc_leaf<BD, Px, SS>(F, Wp, S.big, T, &S.small, (int)(id >> 8), (int)(id & 255), trace);
     }
 }
 

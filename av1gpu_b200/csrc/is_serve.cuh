@@ -254,6 +254,8 @@ int is_serve_submit(is_handle *h, const is_frame *f, int from_host, int *ticket)
     lambda_fx(f->qindex, bd, &F.lam, &F.sqlam);
     F.dcQ = AV1G_T(Dc_Qlookup)[bd == 10][f->qindex];
     F.acQ = AV1G_T(Ac_Qlookup)[bd == 10][f->qindex];
+    F.dcM = quant_recip(F.dcQ);
+    F.acM = quant_recip(F.acQ);
     sl.gen = (sl.gen + 1) & 0x7FFF;
     F.readyQ = S->dQueue;
     F.readyCap = (uint32_t)S->queueCap;

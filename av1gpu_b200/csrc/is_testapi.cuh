@@ -4,7 +4,7 @@
 
 namespace {
 
-struct TestScr { int32_t buf[64 * 65]; int16_t q[1024]; };
+struct TestScr { int32_t buf[64 * 65]; int16_t q[1024]; uint32_t words[EVAL_WORDS]; };
 
 // one warp per block: the search's own grp_eval (one task, 32 lanes) with a residual array as the source; the
 // coefficients are read back from the scratch (quantisation writes only the levels)
@@ -15,9 +15,9 @@ __global__ void k_test_fwd_quant(int n, const int32_t *res, int txSz, int txType
     const int b = blockIdx.x * 2 + (threadIdx.x >> 5);
     if (b >= n) return;
     const int W = txw(txSz), H = txh(txSz), tw = min(W, 32), th = min(H, 32), nc = tw * th, lw = 31 - __clz(W);
-    const EvalIn e{txType, plane, skipCtx, dcCtx, intraDir, dcQ, acQ, rate_tabs_global(qctx)};
+    const EvalIn e{txType, plane, skipCtx, dcCtx, intraDir, dcQ, acQ, quant_recip(dcQ), quant_recip(acQ), rate_tabs_global(qctx)};
     ResFn<uint8_t> rf{nullptr, 0, nullptr, lw, res + (size_t)b * W * H};
-    const EvalOut o = grp_eval<8, uint8_t>(txSz, rf, e, S.buf, S.q, lane_id(), 32);
+    const EvalOut o = grp_eval<8, TABS_GLOBAL, uint8_t>(txSz, rf, e, S.buf, S.q, S.words, lane_id(), 32);
     for (int idx = lane_id(); idx < nc; idx += 32) {
         coef[(size_t)b * nc + idx] = S.buf[(idx / tw) * (W + 1) + idx % tw];
         lv[(size_t)b * nc + idx] = S.q[idx];

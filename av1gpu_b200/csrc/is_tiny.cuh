@@ -359,7 +359,7 @@ __device__ __forceinline__ void tiny_block(const FrameDesc &F, const TinySmem<Px
         int res[N], q[N];
 #pragma unroll
         for (int i = 0; i < N; i++) res[i] = src[i] - (int)((pw[i / PPW] >> (PB * (i % PPW))) & PMASK);
-        const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, T};
+        const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, F.dcM, F.acM, T};
         const EvalOut o = thr_eval<BD, LW, LH>(txSz, res, e, iscan, 32, q);
         return o.D + F.lam * (o.R + c_avgY[m] + overhead);
     };
@@ -668,7 +668,7 @@ __device__ __forceinline__ void mid_block(const FrameDesc &F, MidSmem<Px> &S, co
             for (int i = 0; i < H; i++)
 #pragma unroll
                 for (int j = 0; j < W; j++) res[i * W + j] = (int)src[i * TW + j] - qs[i * W + j];
-            const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, T};
+            const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, F.dcM, F.acM, T};
             const EvalOut o = mid_eval<BD, LW, LH>(txSz, res, e, iscan, 64, qs);
             const i64 J = o.D + F.lam * (o.R + mbits(c) + overhead);
             if (need && job == 29) rank.add(bestJ, AV1G_DCT_DCT);   // the winner's DCT_DCT cost, before its other types

@@ -84,3 +84,22 @@ def test_mixed_format_batch(enc):
         for i, (s, b) in enumerate(zip(singles, batch)):
             assert _same_record(s, b), "image %d of the mixed batch differs (graph %s)" % (i, graph)
     enc.set_batch_options(use_graph=False, front_streams=1)
+
+
+@pytest.mark.parametrize("bd,c444,w,h,q", [(8, False, 72, 136, 1), (8, False, 136, 72, 60), (8, True, 68, 68, 255), (10, False, 72, 72, 2),
+                                           (10, True, 40, 72, 120)])
+def test_formats_noise_levels(enc, bd, c444, w, h, q):
+    """Full-range noise beside a flat half: blocks of every small size with long ends of block, levels above 14 (the packed
+    levels' cap) up to the largest a quantiser step gives, and empty blocks; at the qindex extremes, sizes that cut blocks."""
+    dt, top = (np.uint16, 1023) if bd == 10 else (np.uint8, 255)
+    rng = np.random.default_rng(q)
+    shapes = [(h, w)] + [((h, w) if c444 else ((h + 1) // 2, (w + 1) // 2))] * 2
+    planes = [rng.integers(0, 2, s).astype(dt) * top if i == 0 else rng.integers(0, top + 1, s).astype(dt) for i, s in enumerate(shapes)]
+    for p in planes:
+        p[:, :p.shape[1] // 2] = np.clip(top // 2 + rng.integers(-3, 4, (p.shape[0], p.shape[1] // 2)), 0, top)
+        p[:p.shape[0] // 4] = top // 2
+    g = enc.encode(planes, q)
+    o = O.encode(planes, q, bit_depth=bd, chroma_444=c444)
+    assert np.array_equal(g.blocks.view(np.uint8), o.blocks.view(np.uint8)) and np.array_equal(g.block_txb, o.block_txb)
+    assert np.array_equal(g.txb.view(np.uint8), o.txb.view(np.uint8)) and np.array_equal(g.coeffs, o.coeffs)
+    assert all(np.array_equal(a, b) for a, b in zip(g.recon, o.recon))
