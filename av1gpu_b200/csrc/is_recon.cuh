@@ -212,9 +212,9 @@ __device__ void rc_edges_rec(const FrameDesc &F, int pl, int px, int py, int W, 
     __syncwarp();
 }
 
-// record a finished tx block: eob, culLevel / dc category into the context maps, the txb entry and its levels
-static __device__ __noinline__ int rc_record(const FrameDesc &F, const RateTabs &T, int sb, int plane, int txSz, int txType, int x4, int y4, const int16_t *q,
-                         int txbIdx, int coefOff) {
+// a finished tx block, first part: its eob, culLevel / dc category into the context maps (what later leaves read)
+static __device__ __noinline__ int rc_record_maps(const FrameDesc &F, const RateTabs &T, int plane, int txSz, int txType, int x4, int y4,
+                                                  const int16_t *q) {
     IS_SHARED_PTR(&F); IS_SHARED_PTR(q);
     const int lane = lane_id();
     const int W = txw(txSz), H = txh(txSz), n = min(W, 32) * min(H, 32);
@@ -239,6 +239,13 @@ static __device__ __noinline__ int rc_record(const FrameDesc &F, const RateTabs 
             F.cDc[plane][(size_t)yy * stride + xx] = (uint8_t)(eob ? dcCat : 0);
         }
     }
+    return eob;
+}
+// second part: the txb entry and its levels (only the pack reads them)
+static __device__ __noinline__ void rc_record_out(const FrameDesc &F, int sb, int plane, int txSz, int txType, int x4, int y4, const int16_t *q,
+                                                  int eob, int txbIdx, int coefOff) {
+    IS_SHARED_PTR(&F); IS_SHARED_PTR(q);
+    const int lane = lane_id(), n = min(txw(txSz), 32) * min(txh(txSz), 32);
     int16_t *oc = F.oCoeffs + (size_t)sb * SB_MAX_COEF + coefOff;
 #pragma unroll 2
     for (int i = lane; i < n; i += 32) oc[i] = q[i];
@@ -252,6 +259,11 @@ static __device__ __noinline__ int rc_record(const FrameDesc &F, const RateTabs 
         F.oTxb[(size_t)sb * SB_MAX_TXB + txbIdx] = t;
     }
     __syncwarp();
+}
+__device__ __forceinline__ int rc_record(const FrameDesc &F, const RateTabs &T, int sb, int plane, int txSz, int txType, int x4, int y4,
+                                         const int16_t *q, int txbIdx, int coefOff) {
+    const int eob = rc_record_maps(F, T, plane, txSz, txType, x4, y4, q);
+    rc_record_out(F, sb, plane, txSz, txType, x4, y4, q, eob, txbIdx, coefOff);
     return eob;
 }
 
@@ -500,7 +512,8 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
         return o < li;
     };
     // ================= luma =================
-    int yMode, yDelta, eobY;
+    int yMode, yDelta, eobY, lumaT;
+    const int16_t *lumaQ;
     {
         const int txSz = ST(Max_Tx_Size_Rect)[bsize];
         const int W = txw(txSz), H = txh(txSz), lw = 31 - __clz(W), lh = 31 - __clz(H);
@@ -514,6 +527,8 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int i = lane + 32 * k;
+            ra[k] = rl[k] = (Px)0;
+            if (k && n <= 32 * k) continue;   // (small blocks: one load of each)
             ra[k] = i < n ? ldcg(recY + (size_t)(y - 1) * rp + min(x + i, aLim)) : (Px)0;
             rl[k] = i < n ? ldcg(recY + (size_t)min(y + i, lLim) * rp + x - 1) : (Px)0;
         }
@@ -536,6 +551,7 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int i = lane + 32 * k;
+                if (k && n <= 32 * k) break;
                 if (i < n) {
                     A[i] = availU ? ((!haveAR && i >= W) ? aW : ra[k]) : (availL ? l0 : (Px)((1 << (BD - 1)) - 1));
                     L[i] = availL ? ((!haveBL && i >= H) ? lH : rl[k]) : (availU ? a0 : (Px)((1 << (BD - 1)) + 1));
@@ -699,7 +715,9 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
                 atomicExch(&Big.lock, 0);
             }
         }
-        eobY = rc_record(F, T, sb, 0, txSz, bestT, x >> 2, y >> 2, best, txbBase, coefBase);
+        eobY = rc_record_maps(F, T, 0, txSz, bestT, x >> 2, y >> 2, best);
+        lumaQ = best;
+        lumaT = bestT;
         yMode = bm;
         yDelta = cand_delta(bestC);
         const int lbw = 31 - __clz(bw);
@@ -724,6 +742,8 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
             if (atomicSub(F.depCnt + d, 1) == 1) push_ready(F, d);
         }
     }
+    // off the dependency chain: the luma's txb entry and levels
+    rc_record_out(F, sb, 0, ST(Max_Tx_Size_Rect)[bsize], lumaT, x >> 2, y >> 2, lumaQ, eobY, txbBase, coefBase);
     // ================= chroma =================
     int uv = 0, duv = 0, aU = 0, aV = 0, eobU = 0, eobV = 0;
     if (hasC) {
