@@ -13,6 +13,7 @@
 //   - the levels of a row lie in one word, 4 bits each (capped at 15, and at 3 for the base contexts), so the context
 //     sums of a whole row are a few shifts and additions of words instead of five bounds-checked loads a coefficient;
 //   - the scan position and the position's context offset come from one table load a coefficient.
+// quant_level, row_bits and pos_entry are also the analysis' (k_analysis_tiny, one thread a block).
 #pragma once
 #include "is_dev.cuh"
 
@@ -29,15 +30,19 @@ struct __align__(16) SmallTabs {
     uint16_t pos[SMALL_SIZES][3][64];   // per (size, class, natural position): scan position | context offset << 8
     uint8_t typeIdx[16];                // index of a tx type in TX_SET_INTRA_1
 };
+// entry of scan position c of (size, class): its natural position's scan position | context offset << 8
+__device__ __forceinline__ void pos_entry(uint16_t *tab, const RateTabs &T, int txSz, int cls, int c) {
+    const int p = T.scan[c_scanOff[txSz][cls] + c], row = p >> ST(Tx_Width_Log2)[txSz], col = p & (txw(txSz) - 1);
+    const int off = cls == AV1G_TX_CLASS_2D ? T.baseCtx[txSz * 25 + min(row, 4) * 5 + min(col, 4)]
+                                            : ST(Coeff_Base_Pos_Ctx_Offset)[min(cls == AV1G_TX_CLASS_VERT ? row : col, 2)];
+    tab[p] = (uint16_t)(c | off << 8);
+}
 // all threads of the CTA, after the scans are staged (and a barrier); followed by a barrier
 __device__ __forceinline__ void small_tabs_stage(SmallTabs &S, const RateTabs &T, int tid, int nt) {
     for (int k = tid; k < SMALL_SIZES * 3 * 64; k += nt) {
         const int si = k / 192, cls = (k / 64) % 3, c = k % 64, txSz = small_size(si);
         if (c >= txw(txSz) * txh(txSz)) continue;
-        const int p = T.scan[c_scanOff[txSz][cls] + c], row = p >> ST(Tx_Width_Log2)[txSz], col = p & (txw(txSz) - 1);
-        const int off = cls == AV1G_TX_CLASS_2D ? T.baseCtx[txSz * 25 + min(row, 4) * 5 + min(col, 4)]
-                                                : ST(Coeff_Base_Pos_Ctx_Offset)[min(cls == AV1G_TX_CLASS_VERT ? row : col, 2)];
-        S.pos[si][cls][p] = (uint16_t)(c | off << 8);
+        pos_entry(S.pos[si][cls], T, txSz, cls, c);
     }
     for (int t = tid; t < 16; t += nt) S.typeIdx[t] = (uint8_t)tx_index_in_set(AV1G_TX_SET_INTRA_1, t);
 }
@@ -46,6 +51,74 @@ __device__ __forceinline__ void small_tabs_stage(SmallTabs &S, const RateTabs &T
 // keeps the tasks of a warp on different banks
 template <int LW, int LH> constexpr int small_words() { return 2 * ((1 << LH) + 4) * (LW == 4 ? 2 : 1) + 1; }
 
+template <int LW> using PackedRow = typename std::conditional<LW == 4, unsigned long long, uint32_t>::type;   // 4 bits a column
+
+// bits of the coefficients of row rr of a tx block of 1 << LW columns whose levels are packed 4 bits each: a0 .. a4 the rows
+// rr .. rr + 4 capped at 3, b0 .. b2 the rows rr .. rr + 2 capped at 15 (a3, a4 and b2 are used by the vertical class only).
+// Every sign counts one bit (the caller corrects the DC's).  tab: scan position | context offset << 8 of the row's
+// positions; level(j): the signed level of column j.
+template <int LW, int LH, typename Level>
+__device__ __forceinline__ int row_bits(int rr, PackedRow<LW> a0, PackedRow<LW> a1, PackedRow<LW> a2, PackedRow<LW> a3, PackedRow<LW> a4,
+                                        PackedRow<LW> b0, PackedRow<LW> b1, PackedRow<LW> b2, int cls, int eob, const uint16_t *tab,
+                                        const uint16_t *cBase, const uint16_t *cEob, const uint16_t *cBr, const Level &level) {
+    typedef PackedRow<LW> Row;
+    constexpr int W = 1 << LW, N = 1 << (LW + LH);
+    int b = 0;
+    const bool c2 = cls == AV1G_TX_CLASS_2D, ch = cls == AV1G_TX_CLASS_HORIZ;
+    // the base contexts' neighbours (at most 5 of at most 3: 4 bits a sum), and the third neighbour of the ranges' contexts,
+    // beside (0, 1) and (1, 0)
+    const Row m = (a0 >> 4) + a1 + (c2 ? (a1 >> 4) + (a0 >> 8) + a2 : ch ? (a0 >> 8) + (a0 >> 12) + (a0 >> 16) : a2 + a3 + a4);
+    const Row x2 = c2 ? b1 >> 4 : ch ? b0 >> 8 : b2;
+    // base symbols of the row, without branches: a coefficient past the end of block costs nothing, the last one takes
+    // the end-of-block table
+    Row big = 0;
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+        const int t = tab[j], c = t & 0xFF, l3 = (int)(a0 >> (4 * j)) & 3;
+        int ctx = min(((int)(m >> (4 * j) & 15) + 1) >> 1, 4) + (t >> 8);
+        if (j == 0) ctx = rr == 0 && cls == AV1G_TX_CLASS_2D ? 0 : ctx;
+        const int ectx = c == 0 ? 0 : c <= N / 8 ? 1 : c <= N / 4 ? 2 : 3;
+        // (a valid entry for every coefficient: the last one's level is at least 1)
+        const int bits = *(c == eob - 1 ? cEob + ectx * IS_CD(coeff_base_eob, 3) + l3 - 1 : cBase + ctx * IS_CD(coeff_base, 3) + l3);
+        b += (c < eob ? bits : 0) + (l3 ? 256 : 0);
+        big |= (Row)(l3 > 2 ? 1 : 0) << (4 * j);
+    }
+    // the ranges and remainders of the levels above 2, one after the other
+#pragma unroll 1
+    for (; big; big &= big - 1) {
+        const int sh = LW == 4 ? __ffsll((long long)big) - 1 : __ffs((int)big) - 1, j = sh >> 2;
+        const int l = (int)(b0 >> sh) & 15, right = (int)((b0 >> sh) >> 4) & 15;
+        int mg = right + ((int)(b1 >> sh) & 15) + ((int)(x2 >> sh) & 15);
+        mg = min((mg + 1) >> 1, 6);
+        const int near = cls == AV1G_TX_CLASS_2D ? (rr < 2 && j < 2) : cls == AV1G_TX_CLASS_HORIZ ? j == 0 : rr == 0;
+        const uint16_t *cr = cBr + ((rr | j) == 0 ? mg : near ? mg + 7 : mg + 14) * IS_CD(coeff_br, 3);
+        const int rem = l - 3, full = (rem * 11) >> 5;   // rem / 3: at most 4 symbols
+        b += full * cr[3];
+        if (full < 4) b += cr[rem - 3 * full];
+        if (l == 15) {
+            const int v = abs(level(j));
+            if (v > 14) b += (2 * (31 - __clz(v - 14)) + 1) * 256;
+        }
+    }
+    return b;
+}
+
+// level of a coefficient, its distance from the dequantised value and its packed forms (tx sizes of dequantisation
+// denominator 1); no branch: the coefficients of a row are independent chains.  M: quant_recip(step)
+template <int BD>
+__device__ __forceinline__ int quant_level(int v, int step, uint32_t M, i64 &dist) {
+    const int a = abs(v), St = step << FB;
+    const uint32_t n = (uint32_t)(8 * a + 3 * St), d = (uint32_t)(8 * St);
+    uint32_t u = __umulhi(n, M);   // n / d or one less
+    u += n - u * d >= d;
+    const int l = a * 32 >= 21 * St ? min((int)u, 16383) : 0;
+    // |dequantised|: 24 bits, clamped to 2^(7 + BD) below and one less above zero
+    const int dq = min((l * step) & 0xFFFFFF, (1 << (7 + BD)) - (v >= 0 ? 1 : 0));
+    const int df = a - dq * (1 << FB);
+    dist += (i64)df * df;
+    return v < 0 ? -l : l;
+}
+
 // One evaluation by lanes g = 0, 1 of a pair (all lanes of the warp call it together): src and pred are W x H in shared
 // memory, rows are small_words() words of scratch and q the W x H levels of the task.  dcM / acM: floor(2^32 / (64 step)).
 template <int BD, int LW, int LH, typename Px>
@@ -53,7 +126,7 @@ __device__ __forceinline__ EvalOut small_eval(int si, const Px *src, const Px *p
                                               int dcQ, int acQ, uint32_t dcM, uint32_t acM, const uint16_t *C, const SmallTabs &S,
                                               int32_t *buf, uint32_t *rows, int16_t *q, int g) {
     constexpr int W = 1 << LW, H = 1 << LH, N = W * H, CW = W / 2, RH = H / 2;
-    typedef typename std::conditional<LW == 4, unsigned long long, uint32_t>::type Row;   // 4 bits a column
+    typedef PackedRow<LW> Row;
     const int txSz = LW == LH ? (LW == 2 ? AV1G_TX_4X4 : AV1G_TX_8X8) : LW == 2 ? (LH == 3 ? AV1G_TX_4X8 : AV1G_TX_4X16)
                    : LW == 3 ? AV1G_TX_8X4 : AV1G_TX_16X4;
     constexpr int rowShift = small_row_shift(LW, LH);
@@ -94,18 +167,8 @@ __device__ __forceinline__ EvalOut small_eval(int si, const Px *src, const Px *p
             if (rect) v = (v * 5793 + 2048) >> 12;
             if constexpr (s2 > 0) v = (v + (1 << (s2 - 1))) >> s2;
             else v = v * (1 << -s2);
-            // no branch: the coefficients of a row are independent chains
             const bool dc = j == 0 && rr == 0;
-            const int step = dc ? dcQ : acQ, a = abs(v), St = step << FB;
-            const uint32_t n = (uint32_t)(8 * a + 3 * St), d = (uint32_t)(8 * St);
-            uint32_t u = __umulhi(n, dc ? dcM : acM);   // n / d or one less
-            u += n - u * d >= d;
-            const int l = a * 32 >= 21 * St ? min((int)u, 16383) : 0;
-            const int qv = v < 0 ? -l : l;
-            // |dequantised|: 24 bits, clamped to 2^(7 + BD) below and one less above zero
-            const int dq = min((l * step) & 0xFFFFFF, (1 << (7 + BD)) - (v >= 0 ? 1 : 0));
-            const int df = a - dq * (1 << FB);
-            dist += (i64)df * df;
+            const int qv = quant_level<BD>(v, dc ? dcQ : acQ, dc ? dcM : acM, dist), l = abs(qv);
             eob = max(eob, l ? (int)(tab[rr * W + j] & 0xFF) + 1 : 0);
             p3 |= (Row)min(l, 3) << (4 * j);
             p15 |= (Row)min(l, 15) << (4 * j);
@@ -141,47 +204,9 @@ __device__ __forceinline__ EvalOut small_eval(int si, const Px *src, const Px *p
         for (int i = 0; i < RH; i++) {
             const int rr = g * RH + i;
             const Row a0 = get(rr), a1 = get(rr + 1), a2 = get(rr + 2), b0 = get(H + 4 + rr), b1 = get(H + 4 + rr + 1);
-            Row m = (a0 >> 4) + a1;   // the base contexts' neighbours (at most 5 of at most 3: 4 bits a sum)
-            Row x2;                   // and the third neighbour of the ranges' contexts, beside (0, 1) and (1, 0)
-            if (cls == AV1G_TX_CLASS_2D) { m += (a1 >> 4) + (a0 >> 8) + a2; x2 = b1 >> 4; }
-            else if (cls == AV1G_TX_CLASS_HORIZ) { m += (a0 >> 8) + (a0 >> 12) + (a0 >> 16); x2 = b0 >> 8; }
-            else { m += a2 + get(rr + 3) + get(rr + 4); x2 = get(H + 4 + rr + 2); }
-            // base symbols of the row, without branches: a coefficient past the end of block costs nothing, the last one
-            // takes the end-of-block table
-#pragma unroll
-            for (int j = 0; j < W; j++) {
-                const int t = tab[rr * W + j], c = t & 0xFF, l3 = (int)(a0 >> (4 * j)) & 3;
-                int ctx = min(((int)(m >> (4 * j) & 15) + 1) >> 1, 4) + (t >> 8);
-                if (j == 0) ctx = rr == 0 && cls == AV1G_TX_CLASS_2D ? 0 : ctx;
-                const int ectx = c == 0 ? 0 : c <= N / 8 ? 1 : c <= N / 4 ? 2 : 3;
-                const uint16_t *e = c == eob - 1 ? cEob + ectx * IS_CD(coeff_base_eob, 3) + l3 - 1 : cBase + ctx * IS_CD(coeff_base, 3) + l3;
-                const int bits = *(c < eob ? e : cBase);
-                b += c < eob ? bits : 0;
-            }
-            // signs: one bit each; the ranges and remainders of the levels above 2, one after the other
-            Row big = 0;
-#pragma unroll
-            for (int j = 0; j < W; j++) {
-                const int l = (int)(b0 >> (4 * j)) & 15;
-                b += l ? 256 : 0;
-                big |= (Row)(l > 2 ? 1 : 0) << (4 * j);
-            }
-#pragma unroll 1
-            for (; big; big &= big - 1) {
-                const int sh = LW == 4 ? __ffsll((long long)big) - 1 : __ffs((int)big) - 1, j = sh >> 2, pos = rr * W + j;
-                const int l = (int)(b0 >> sh) & 15, right = (int)((b0 >> sh) >> 4) & 15;
-                int mg = right + ((int)(b1 >> sh) & 15) + ((int)(x2 >> sh) & 15);
-                mg = min((mg + 1) >> 1, 6);
-                const int near = cls == AV1G_TX_CLASS_2D ? (rr < 2 && j < 2) : cls == AV1G_TX_CLASS_HORIZ ? j == 0 : rr == 0;
-                const uint16_t *cr = cBr + (pos == 0 ? mg : near ? mg + 7 : mg + 14) * IS_CD(coeff_br, 3);
-                const int rem = l - 3, full = (rem * 11) >> 5;   // rem / 3
-                b += full * cr[3];
-                if (full < 4) b += cr[rem - 3 * full];
-                if (l == 15) {
-                    const int v = abs((int)q[pos]);
-                    if (v > 14) b += (2 * (31 - __clz(v - 14)) + 1) * 256;
-                }
-            }
+            b += row_bits<LW, LH>(rr, a0, a1, a2, cls == AV1G_TX_CLASS_VERT ? get(rr + 3) : 0, cls == AV1G_TX_CLASS_VERT ? get(rr + 4) : 0, b0, b1,
+                                  cls == AV1G_TX_CLASS_VERT ? get(H + 4 + rr + 2) : 0, cls, eob, tab + rr * W, cBase, cEob, cBr,
+                                  [&](int j) -> int { return q[rr * W + j]; });
         }
         if (g == 0 && q[0]) b += C[ci_dc_sign(ptype, dcCtx) + (q[0] < 0)] - 256;   // the DC sign has its own contexts
     }

@@ -11,15 +11,25 @@
 //   kept with their predictions (insertion in cost order, earlier candidate first on ties), exact-rate RD of the top 4
 //   with DCT_DCT, then the other tx types of the set for the winner.
 // One CTA of 256 threads per SB: the 256 4x4 blocks, then the 128 4x8 (warps 0-3) and 128 8x4 blocks (warps 4-7).
+//
+// Bound by instruction issue (and, at this code size, by instruction fetch): no DRAM traffic beside the tile.  So the
+// levels are quantised without a division (quant_level) and, in k_analysis_tiny, packed 4 bits each into one register a
+// row, whose shifts give the context sums of the whole row (row_bits) instead of eight bounds-checked neighbours a
+// coefficient.  In k_analysis_mid the levels stay in shared memory and the rate is coeff_bits over the scan positions: the
+// loop ends with the block's last level, and most blocks have few.  Both, with the slots' strides below: the analysis of a
+// 4000x3000 picture 70.0 -> 66.6 ms, 1920x1080 13.4 -> 11.8, 160x120 1.92 -> 1.66, the front end of 16 pictures of 256 to
+// 2048 samples a side with learned shortlists 128 -> 107 ms.
 #pragma once
 #include "is_dev.cuh"
 #include "is_frame.cuh"
 #include "is_analysis.cuh"
+#include "is_small.cuh"
 
 namespace is {
 
-// Spec constants used as compile-time indices: Sig_Ref_Diff_Offset, Mag_Ref_Offset_With_Tx_Class (spec 8.3.2 / the
-// av1core tables; the library checks them against av1core's at upload) and Dr_Intra_Derivative at 23, 45, 67 degrees.
+// Spec constants fixed at compile time (the library checks them against av1core's tables at upload): Sig_Ref_Diff_Offset and
+// Mag_Ref_Offset_With_Tx_Class (spec 8.3.2), which the row and column shifts of packed levels (row_bits, grp_eval_x) spell
+// out, and Dr_Intra_Derivative at 23, 45, 67 degrees.
 // (row, column) offset d of neighbour k for tx class c (0 2D, 1 HORIZ, 2 VERT)
 __host__ __device__ constexpr int sig_ref(int c, int k, int d) {
     return k == 0 ? (d == 0 ? 0 : 1) : k == 1 ? (d == 0 ? 1 : 0)
@@ -36,7 +46,8 @@ constexpr int TINY_THREADS = 256;
 template <typename Px> struct TinySmem {      // Px: the sample type (uint8_t 8-bit, uint16_t 10-bit)
     static constexpr int TW = 144, TH = 65;   // the SB tile of the analysis (columns sbx-16 .., rows sby-1 ..)
     Px tile[TH * TW];
-    uint8_t iscan[3][3][32];                  // scan position of each coefficient: (4x4, 4x8, 8x4) x (2D, HORIZ, VERT)
+    uint16_t pos[3][3][32];                   // scan position | context offset << 8 of each coefficient: (4x4, 4x8, 8x4) x
+                                              // (2D, HORIZ, VERT)
     RateStage T;
 };
 
@@ -117,70 +128,32 @@ __device__ __forceinline__ void tpred(const int *A, const int *L, int dcv, int *
     }
 }
 
-// ---- rate of the levels q (natural order) of a 4- or 8-point tx block of class CLS: coeff_bits over the scan
-// positions c < eob, walked in natural order through the inverse scan ----
-template <int LW, int LH, int CLS>
-__device__ __forceinline__ int tcoeff_rate(const int *q, const uint8_t *iscan, int eob, int txSz, int ptype, int dcCtx, const RateTabs &T) {
-    constexpr int W = 1 << LW, H = 1 << LH, N = W * H;
-    const uint16_t *C = T.cost;
-    const int txSzCtx = (ST(Tx_Size_Sqr)[txSz] + ST(Tx_Size_Sqr_Up)[txSz] + 1) >> 1;
+// ---- rate of a tx block whose packed rows are in registers (p3 / p15: H rows and 4 rows of zeros below): row_bits over
+// the rows, the DC sign, txb_skip, tx type and eob position ----
+template <int LW, int LH, typename Level>
+__device__ __forceinline__ i64 thr_rate(int txSz, const EvalIn &e, int eob, const PackedRow<LW> *p3, const PackedRow<LW> *p15, const uint16_t *pos,
+                                        int cls, int dcLevel, const Level &level) {
+    constexpr int W = 1 << LW, H = 1 << LH;
     int b = 0;
+    if (eob) {
+        const int ptype = e.plane > 0;
+        const int txSzCtx = (ST(Tx_Size_Sqr)[txSz] + ST(Tx_Size_Sqr_Up)[txSz] + 1) >> 1;
+        const uint16_t *C = e.T.cost;
+        const uint16_t *cBase = C + ci_base(txSzCtx, ptype, 0), *cBr = C + ci_br(min(txSzCtx, (int)AV1G_TX_32X32), ptype, 0);
+        const uint16_t *cEob = C + ci_base_eob(txSzCtx, ptype, 0);
 #pragma unroll
-    for (int pos = 0; pos < N; pos++) {
-        const int c = iscan[pos];
-        if (c >= eob) continue;
-        const int row = pos >> LW, col = pos & (W - 1);
-        const int qv = q[pos], v = abs(qv), level = min(v, 15);
-        int bb;
-        if (c == eob - 1) {
-            const int bctx = c == 0 ? 0 : c <= N / 8 ? 1 : c <= N / 4 ? 2 : 3;
-            bb = C[ci_base_eob(txSzCtx, ptype, bctx) + min(level, 3) - 1];
-        } else {
-            int mag = 0;
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                const int rr = row + sig_ref(CLS, k, 0), cc = col + sig_ref(CLS, k, 1);
-                if (rr < H && cc < W) mag += min(abs(q[rr * W + cc]), 3);
-            }
-            int bctx = min((mag + 1) >> 1, 4);
-            if (CLS == AV1G_TX_CLASS_2D) bctx = pos == 0 ? 0 : bctx + T.baseCtx[txSz * 25 + min(row, 4) * 5 + min(col, 4)];
-            else bctx += ST(Coeff_Base_Pos_Ctx_Offset)[min(CLS == AV1G_TX_CLASS_VERT ? row : col, 2)];
-            bb = C[ci_base(txSzCtx, ptype, bctx) + min(level, 3)];
-        }
-        if (level > 2) {
-            int mag = 0;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const int rr = row + mag_ref(CLS, k, 0), cc = col + mag_ref(CLS, k, 1);
-                if (rr < H && cc < W) mag += min(abs(q[rr * W + cc]), 15);
-            }
-            mag = min((mag + 1) >> 1, 6);
-            const int brctx = pos == 0 ? mag
-                            : CLS == AV1G_TX_CLASS_2D ? ((row < 2 && col < 2) ? mag + 7 : mag + 14)
-                            : CLS == AV1G_TX_CLASS_HORIZ ? (col == 0 ? mag + 7 : mag + 14) : (row == 0 ? mag + 7 : mag + 14);
-            const int cid = ci_br(min(txSzCtx, (int)AV1G_TX_32X32), ptype, brctx);
-            int rem = level - 3;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int k = min(rem, 3);
-                bb += C[cid + k];
-                rem -= k;
-                if (k < 3) break;
-            }
-        }
-        if (v) {
-            bb += c == 0 ? C[ci_dc_sign(ptype, dcCtx) + (qv < 0)] : 256;
-            if (v > 14) bb += (2 * (31 - __clz(v - 14)) + 1) * 256;
-        }
-        b += bb;
+        for (int r = 0; r < H; r++)
+            b += row_bits<LW, LH>(r, p3[r], p3[r + 1], p3[r + 2], p3[r + 3], p3[r + 4], p15[r], p15[r + 1], p15[r + 2], cls, eob, pos + r * W, cBase,
+                                  cEob, cBr, [&](int j) -> int { return level(r * W + j); });
+        if (dcLevel) b += C[ci_dc_sign(ptype, e.dcCtx) + (dcLevel < 0)] - 256;   // the DC sign has its own contexts
     }
-    return b;
+    return b + base_bits_inl(txSz, e, eob);
 }
 
 // ---- one evaluation by one thread (grp_eval's arithmetic for a 4- or 8-point tx size): forward transform of the
 // residual, dead-zone quantisation into q, transform-domain distortion, exact rate ----
 template <int BD, int LW, int LH>
-__device__ __forceinline__ EvalOut thr_eval(int txSz, const int *res, const EvalIn &e, const uint8_t *iscan, int istride, int *q) {
+__device__ __forceinline__ EvalOut thr_eval(int txSz, const int *res, const EvalIn &e, const uint16_t *posTab) {
     constexpr int W = 1 << LW, H = 1 << LH, N = W * H;
     const int rowShift = ST(Transform_Row_Shift)[txSz];
     constexpr int rect = (LW - LH == 1 || LH - LW == 1) ? 1 : 0;
@@ -212,32 +185,25 @@ __device__ __forceinline__ EvalOut thr_eval(int txSz, const int *res, const Eval
         }
     }
     const int cls = e.txType == AV1G_IDTX ? AV1G_TX_CLASS_2D : tx_class(e.txType);
-    const uint8_t *isc = iscan + cls * istride;
+    const uint16_t *pos = posTab + cls * 32;
     i64 dist = 0;
     int eob = 0;
+    PackedRow<LW> p3[H + 4] = {}, p15[H + 4] = {};
 #pragma unroll
     for (int idx = 0; idx < N; idx++) {
-        const int v = buf[idx];
-        const int step = idx == 0 ? e.dcQ : e.acQ;
-        const int a = abs(v), S = step << FB;   // dequantisation denominator 1 for these sizes
-        int l = 0;
-        if (a * 32 >= 21 * S) l = min((8 * a + 3 * S) / (8 * S), 16383);
-        const int qv = v < 0 ? -l : l;
-        q[idx] = qv;
-        const int dq = l ? dequant<BD>(qv, step, 1) * (1 << FB) : 0;
-        const i64 df = (i64)(v - dq);
-        dist += df * df;
-        if (qv) eob = max(eob, isc[idx] + 1);
-    }
-    int b = 0;
-    if (eob) {
-        const int ptype = e.plane > 0;
-        if (cls == AV1G_TX_CLASS_2D) b = tcoeff_rate<LW, LH, AV1G_TX_CLASS_2D>(q, isc, eob, txSz, ptype, e.dcCtx, e.T);
-        else if (cls == AV1G_TX_CLASS_HORIZ) b = tcoeff_rate<LW, LH, AV1G_TX_CLASS_HORIZ>(q, isc, eob, txSz, ptype, e.dcCtx, e.T);
-        else b = tcoeff_rate<LW, LH, AV1G_TX_CLASS_VERT>(q, isc, eob, txSz, ptype, e.dcCtx, e.T);
+        const int qv = quant_level<BD>(buf[idx], idx == 0 ? e.dcQ : e.acQ, idx == 0 ? e.dcM : e.acM, dist), l = abs(qv);
+        buf[idx] = qv;
+        eob = max(eob, l ? (int)(pos[idx] & 0xFF) + 1 : 0);
+        p3[idx >> LW] |= (PackedRow<LW>)min(l, 3) << (4 * (idx & (W - 1)));
+        p15[idx >> LW] |= (PackedRow<LW>)min(l, 15) << (4 * (idx & (W - 1)));
     }
     EvalOut o;
-    o.R = b + base_bits_inl(txSz, e, eob);
+    o.R = thr_rate<LW, LH>(txSz, e, eob, p3, p15, pos, cls, buf[0], [&](int at) -> int {
+        int v = 0;   // (a level of 15 or more: the registers are searched)
+#pragma unroll
+        for (int k = 0; k < N; k++) v = k == at ? buf[k] : v;
+        return v;
+    });
     o.D = dist << dsh;
     o.eob = eob;
     return o;
@@ -354,13 +320,13 @@ __device__ __forceinline__ void tiny_block(const FrameDesc &F, const TinySmem<Px
     // ---- RD: the top 4 with DCT_DCT, then the other types of the set for the winner (first of equal costs wins) ----
     const bool hasC = has_chroma(bs, y >> 2, x >> 2, F.ssx);
     const int overhead = (hasC ? UV_OVERHEAD : 0) + c_avgSkip0;
-    const uint8_t *iscan = &S.iscan[sizeIdx][0][0];
+    const uint16_t *posTab = &S.pos[sizeIdx][0][0];
     auto rd = [&](const uint32_t *pw, int m, int t) -> i64 {
-        int res[N], q[N];
+        int res[N];
 #pragma unroll
         for (int i = 0; i < N; i++) res[i] = src[i] - (int)((pw[i / PPW] >> (PB * (i % PPW))) & PMASK);
         const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, F.dcM, F.acM, T};
-        const EvalOut o = thr_eval<BD, LW, LH>(txSz, res, e, iscan, 32, q);
+        const EvalOut o = thr_eval<BD, LW, LH>(txSz, res, e, posTab);
         return o.D + F.lam * (o.R + c_avgY[m] + overhead);
     };
     i64 bestJ = INF;
@@ -436,7 +402,7 @@ __global__ void __launch_bounds__(TINY_THREADS, BD == 8 ? 2 : 1) k_analysis_tiny
     for (int k = tid; k < 3 * 3 * 32; k += TINY_THREADS) {
         const int si = k / 96, cls = (k / 32) % 3, c = k % 32;
         const int txSz = si == 0 ? AV1G_TX_4X4 : si == 1 ? AV1G_TX_4X8 : AV1G_TX_8X4;
-        if (c < (si == 0 ? 16 : 32)) S.iscan[si][cls][T.scan[c_scanOff[txSz][cls] + c]] = (uint8_t)c;
+        if (c < (si == 0 ? 16 : 32)) pos_entry(S.pos[si][cls], T, txSz, cls, c);
     }
     __syncthreads();
     int tc = 0, tr = 0;
@@ -470,9 +436,11 @@ constexpr int MID_SBS = 3, MID_THREADS = 64 * MID_SBS;
 template <typename Px> struct MidSmem {   // Px: the sample type
     static constexpr int TW = 144, TH = 65;
     Px tile[MID_SBS][TH * TW];
-    uint8_t iscan[3][64];                // the shape's tx size x (2D, HORIZ, VERT)
-    Px edge[MID_THREADS][2][24];         // per thread: AboveRow[-1 .. 22], LeftCol[-1 .. 22]
-    int16_t q[MID_THREADS][64];          // per thread: levels of the evaluation in progress
+    uint16_t pos[3][64];                 // scan position | context offset << 8: the shape's tx size x (2D, HORIZ, VERT)
+    // per thread: AboveRow[-1 .. 22], LeftCol[-1 .. 22]; levels of the evaluation in progress.  Strides of an odd number of
+    // words: the threads of a warp read and write the same index of their slots, on 32 banks
+    Px edge[MID_THREADS][2][sizeof(Px) == 1 ? 26 : 25];
+    int16_t q[MID_THREADS][66];
     RateStage T;
 };
 
@@ -512,7 +480,7 @@ __device__ __forceinline__ void thr_fwd(int txSz, int txType, const int *res, in
 // one evaluation of a <= 16-point-side block by one thread: transform in registers, levels to qs (shared memory),
 // rate by coeff_bits over the scan
 template <int BD, int LW, int LH>
-__device__ __forceinline__ EvalOut mid_eval(int txSz, const int *res, const EvalIn &e, const uint8_t *iscan, int istride, int16_t *qs) {
+__device__ __forceinline__ EvalOut mid_eval(int txSz, const int *res, const EvalIn &e, const uint16_t *posTab, int16_t *qs) {
     constexpr int W = 1 << LW, H = 1 << LH, N = W * H;
     int buf[N];
     thr_fwd<BD, LW, LH>(txSz, e.txType, res, buf);
@@ -520,22 +488,14 @@ __device__ __forceinline__ EvalOut mid_eval(int txSz, const int *res, const Eval
     constexpr int rect = (LW - LH == 1 || LH - LW == 1) ? 1 : 0;
     const int dsh = 16 - 2 * FB - (2 * (rowShift + 4) - (LW + LH - 2) + rect);
     const int cls = e.txType == AV1G_IDTX ? AV1G_TX_CLASS_2D : tx_class(e.txType);
-    const uint8_t *isc = iscan + cls * istride;
+    const uint16_t *pos = posTab + cls * 64;
     i64 dist = 0;
     int eob = 0;
 #pragma unroll
     for (int idx = 0; idx < N; idx++) {
-        const int v = buf[idx];
-        const int step = idx == 0 ? e.dcQ : e.acQ;
-        const int a = abs(v), S = step << FB;   // dequantisation denominator 1 for these sizes
-        int l = 0;
-        if (a * 32 >= 21 * S) l = min((8 * a + 3 * S) / (8 * S), 16383);
-        const int qv = v < 0 ? -l : l;
+        const int qv = quant_level<BD>(buf[idx], idx == 0 ? e.dcQ : e.acQ, idx == 0 ? e.dcM : e.acM, dist);
         qs[idx] = (int16_t)qv;
-        const int dq = l ? dequant<BD>(qv, step, 1) * (1 << FB) : 0;
-        const i64 df = (i64)(v - dq);
-        dist += df * df;
-        if (qv) eob = max(eob, isc[idx] + 1);
+        eob = max(eob, qv ? (int)(pos[idx] & 0xFF) + 1 : 0);
     }
     const uint16_t *scan = get_scan(e.T, txSz, e.txType);
     int b = 0;
@@ -581,7 +541,7 @@ __device__ __forceinline__ void mid_block(const FrameDesc &F, MidSmem<Px> &S, co
     };
     const bool hasC = has_chroma(bs, y >> 2, x >> 2, F.ssx);
     const int overhead = (hasC ? UV_OVERHEAD : 0) + c_avgSkip0;
-    const uint8_t *iscan = &S.iscan[0][0];
+    const uint16_t *posTab = &S.pos[0][0];
     int16_t *qs = S.q[tid];
     i64 topJ[4] = {INF, INF, INF, INF};
     int topC[4] = {0, 0, 0, 0};
@@ -669,7 +629,7 @@ __device__ __forceinline__ void mid_block(const FrameDesc &F, MidSmem<Px> &S, co
 #pragma unroll
                 for (int j = 0; j < W; j++) res[i * W + j] = (int)src[i * TW + j] - qs[i * W + j];
             const EvalIn e{t, 0, 0, 0, m, F.dcQ, F.acQ, F.dcM, F.acM, T};
-            const EvalOut o = mid_eval<BD, LW, LH>(txSz, res, e, iscan, 64, qs);
+            const EvalOut o = mid_eval<BD, LW, LH>(txSz, res, e, posTab, qs);
             const i64 J = o.D + F.lam * (o.R + mbits(c) + overhead);
             if (need && job == 29) rank.add(bestJ, AV1G_DCT_DCT);   // the winner's DCT_DCT cost, before its other types
             if (need && job >= 29) rank.add(J, t);
@@ -722,7 +682,7 @@ __global__ void __launch_bounds__(MID_THREADS, 2) k_analysis_mid(const __grid_co
     __syncthreads();
     for (int k = tid; k < 3 * 64; k += MID_THREADS) {
         const int cls = k / 64, c = k % 64;
-        S.iscan[cls][T.scan[c_scanOff[txSz][cls] + c]] = (uint8_t)c;
+        pos_entry(S.pos[cls], T, txSz, cls, c);
     }
     __syncthreads();
     const int u = tid >> 6, b = tid & 63, sb = sb0 + u;
