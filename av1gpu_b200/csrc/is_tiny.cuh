@@ -18,7 +18,8 @@
 // coefficient.  In k_analysis_mid the levels stay in shared memory and the rate is coeff_bits over the scan positions: the
 // loop ends with the block's last level, and most blocks have few.  Both, with the slots' strides below: the analysis of a
 // 4000x3000 picture 70.0 -> 66.6 ms, 1920x1080 13.4 -> 11.8, 160x120 1.92 -> 1.66, the front end of 16 pictures of 256 to
-// 2048 samples a side with learned shortlists 128 -> 107 ms.
+// 2048 samples a side with learned shortlists 128 -> 102 ms.  (On the 4000x3000 picture, whose blocks have few levels, contexts
+// looked up per coefficient in k_analysis_tiny take 2.3 ms less; on the batch they take 15 ms more.)
 #pragma once
 #include "is_dev.cuh"
 #include "is_frame.cuh"
@@ -131,7 +132,7 @@ __device__ __forceinline__ void tpred(const int *A, const int *L, int dcv, int *
 // ---- rate of a tx block whose packed rows are in registers (p3 / p15: H rows and 4 rows of zeros below): row_bits over
 // the rows, the DC sign, txb_skip, tx type and eob position ----
 template <int LW, int LH, typename Level>
-__device__ __forceinline__ i64 thr_rate(int txSz, const EvalIn &e, int eob, const PackedRow<LW> *p3, const PackedRow<LW> *p15, const uint16_t *pos,
+__device__ __forceinline__ i64 thr_rate(int txSz, const EvalIn &e, int eob, PackedRow<LW> *p3, PackedRow<LW> *p15, const uint16_t *pos,
                                         int cls, int dcLevel, const Level &level) {
     constexpr int W = 1 << LW, H = 1 << LH;
     int b = 0;
@@ -141,10 +142,18 @@ __device__ __forceinline__ i64 thr_rate(int txSz, const EvalIn &e, int eob, cons
         const uint16_t *C = e.T.cost;
         const uint16_t *cBase = C + ci_base(txSzCtx, ptype, 0), *cBr = C + ci_br(min(txSzCtx, (int)AV1G_TX_32X32), ptype, 0);
         const uint16_t *cEob = C + ci_base_eob(txSzCtx, ptype, 0);
+        // one copy of a row's code, the rows moving down the registers: unrolled, a 4000x3000 picture took 0.2 ms more and the
+        // front end of the batch named above 103.2 instead of 101.6 ms
+#pragma unroll 1
+        for (int r = 0; r < H; r++) {
+            b += row_bits<LW, LH>(r, p3[0], p3[1], p3[2], p3[3], p3[4], p15[0], p15[1], p15[2], cls, eob, pos + r * W, cBase, cEob, cBr,
+                                  [&](int j) -> int { return level(r * W + j); });
 #pragma unroll
-        for (int r = 0; r < H; r++)
-            b += row_bits<LW, LH>(r, p3[r], p3[r + 1], p3[r + 2], p3[r + 3], p3[r + 4], p15[r], p15[r + 1], p15[r + 2], cls, eob, pos + r * W, cBase,
-                                  cEob, cBr, [&](int j) -> int { return level(r * W + j); });
+            for (int k = 0; k + 1 < H + 4; k++) {
+                p3[k] = p3[k + 1];
+                p15[k] = p15[k + 1];
+            }
+        }
         if (dcLevel) b += C[ci_dc_sign(ptype, e.dcCtx) + (dcLevel < 0)] - 256;   // the DC sign has its own contexts
     }
     return b + base_bits_inl(txSz, e, eob);
