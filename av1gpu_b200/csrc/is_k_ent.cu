@@ -5,12 +5,12 @@
 //
 // Every context of the intra syntax is a function of the record alone (neighbouring blocks' sizes, modes and skip
 // flags, neighbouring tx blocks' cumulative levels and DC signs), never of the adapted CDF values, so the symbols are
-// made in parallel and only the range coder with its CDF adaptation runs in order, per tile:
+// made in parallel; a CDF's adaptation runs in order over that CDF's symbols, the range coder over chunks of steps:
 //   k_ent_blocks  one thread per block: the 4x4 mode-info maps (size, luma mode, skip), each SB's first block, the
 //                 owner block of each tx block
 //   k_ent_txb     one thread per tx block: end of block, cumulative level and DC category (into per-plane 4x4 maps),
 //                 the number of its coefficient symbols
-//   k_ent_sb      one thread per SB: the partition walk over its blocks (partition symbols with their contexts) and
+//   k_ent_sb      one warp per SB: the partition walk over its blocks (partition symbols with their contexts) and
 //                 each block's mode-info symbols, into a fixed slot of the block
 //   scans         exclusive sums of the blocks' and tx blocks' symbol counts: where each block's and tx block's
 //                 symbols start in the batch's stream, which is in bitstream order
