@@ -34,7 +34,8 @@ constexpr int RC_BUF_INTS = 1088;
 constexpr int LEAF_WAIT_ITERS = 1 << 20;
 // closed-loop trace (is_set_trace): per queued leaf, globaltimer ns at: 0 slot claimed, 1 slot read, 2 luma prologue
 // done (loads, edges, contexts), 3 luma pass 1 done, 4 pass 2 done, 5 luma published, 6 chroma waits done, 7 chroma
-// screening and RD done, 8 leaf done; 9 the queue entry (image << 32 | sb << 8 | leaf)
+// screening and RD done, 8 leaf done; 9 the queue entry (image << 32 | sb << 8 | leaf).  A pass that does not run has the
+// stamp of what came before it; 6 and 7 are 0 for a leaf without chroma.
 constexpr int TRACE_STAMPS = 10;
 constexpr long long READY_WAIT_NS = 4000000000ll;
 
@@ -644,6 +645,7 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
             // of equal costs wins); the round's winner, if it beats the best so far, leaves its levels in `best`.  Both
             // passes go through one copy of the loop; their tasks lie in Wp.cand (candidate << 4 | type).
             if (skip1) { bestC = br.cand[0]; bestT = AV1G_DCT_DCT; }
+            if (trace && lane == 0) trace[3] = trace[4] = gtimer();   // (a pass that does not run takes no time)
             int curG = 0;
 #pragma unroll 1
             for (int pass = skip1 ? 1 : 0; pass < (set != AV1G_TX_SET_DCTONLY ? 2 : 1); pass++) {
@@ -693,7 +695,10 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
                     }
                     __syncwarp();
                 }
-                if (trace && lane == 0) trace[3 + pass] = gtimer();
+                if (trace && lane == 0) {
+                    trace[4] = gtimer();
+                    if (pass == 0) trace[3] = trace[4];
+                }
             }
         }
         // the winner's prediction (whole warp) for its levels (single-candidate case) and the reconstruction
@@ -1152,6 +1157,7 @@ __global__ void __launch_bounds__(rc_warps_of<BD, SS>() * 32, 1) k_recon(const F
                 if (traceBase) {
                     unsigned long long *tr = traceBase + (size_t)h * TRACE_STAMPS;
                     tr[0] = t0; tr[1] = gtimer(); tr[9] = e - 1;
+                    tr[6] = tr[7] = 0;   // stay so for a leaf without chroma
                 }
             }
         }

@@ -579,7 +579,8 @@ class Encoder:
     def trace(self):
         """Per queued leaf of the last encode (queue order; in a batch, image 0's format group), 10 values: globaltimer ns
         at slot claimed, slot read, luma prologue done, luma pass 1 done, pass 2 done, luma published, chroma waits done,
-        chroma RD done, leaf done; then the queue entry (image << 32 | sb << 8 | leaf)."""
+        chroma RD done, leaf done; then the queue entry (image << 32 | sb << 8 | leaf).  A leaf without chroma has 0 for its
+        chroma values."""
         k = self.TRACE_STAMPS
         n = C.c_uint32()
         self._check(self.L.is_get_trace(self.h, None, 0, C.byref(n)), "is_get_trace")

@@ -275,8 +275,10 @@ int is_debug_tables(is_handle *h, int qctx, uint16_t *cost, size_t cap, int32_t 
 /* Closed-loop trace (debug): is_set_trace(h, 1) before an encode records, per queued leaf (queue order), 10 values:
  * the globaltimer (ns) when a worker claimed its queue slot, read the slot, finished the luma prologue (loads, edges,
  * contexts), luma pass 1, luma pass 2, published the luma, finished its chroma waits, the chroma screening and RD, and
- * the leaf; then the queue entry (image << 32 | sb << 8 | leaf).  The queue is image 0's: in a batch, that of image 0's
- * format group (every image of the group).  is_get_trace copies up to cap / 10 leaves and sets n to the queue's leaves. */
+ * the leaf; then the queue entry (image << 32 | sb << 8 | leaf).  A luma pass that does not run takes no time of its own;
+ * the two chroma values of a leaf without chroma are 0; the six small tx sizes run both passes as one, and both values are
+ * its end.  The queue is image 0's: in a batch, that of image 0's format group (every image of the group).  is_get_trace
+ * copies up to cap / 10 leaves and sets n to the queue's leaves. */
 int is_set_trace(is_handle *h, int on);
 int is_get_trace(is_handle *h, unsigned long long *out, size_t cap, uint32_t *n);
 
