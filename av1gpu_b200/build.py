@@ -5,6 +5,7 @@
 The library includes av1core's public headers (the DecisionRecord ABI, the AV1 spec tables and the default CDFs) from
 AV1CORE_INCLUDE (default: the reference checkout's av1core/include); nothing else of the reference is compiled into it.
 """
+import hashlib
 import os
 import shutil
 import subprocess
@@ -15,7 +16,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libisearch.so")
 # the reference checkout (its av1core headers and sources); set AV1GPU_REF, or AV1CORE_INCLUDE for the headers only.
-# Without it the prebuilt libisearch.so / oracle/_ref are used as they are.
+# Without it the prebuilt libisearch.so / oracle/_ref are used as they are (the build says so).
 REF = os.environ.get("AV1GPU_REF", "")
 AV1CORE_INCLUDE = os.environ.get("AV1CORE_INCLUDE", os.path.join(REF, "av1core", "include") if REF else "")
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
@@ -67,18 +68,46 @@ def _local_deps(src, seen=None):
     return seen
 
 
+def _headers_id():
+    """A digest of av1core's headers, by content: the tables in the library are theirs, and a checkout's dates say nothing."""
+    h = hashlib.sha256()
+    for d, dirs, files in os.walk(AV1CORE_INCLUDE):
+        dirs.sort()
+        for f in sorted(files):
+            path = os.path.join(d, f)
+            with open(path, "rb") as fh:
+                data = fh.read()
+            h.update(("%s %d\n" % (os.path.relpath(path, AV1CORE_INCLUDE), len(data))).encode() + data)
+    return h.hexdigest()
+
+
+def _built_from():
+    """The headers' digest the objects and the library were compiled from; empty when that is not known."""
+    try:
+        with open(os.path.join(BUILD_DIR, "headers.id")) as f:
+            return f.read().strip()
+    except OSError:
+        return ""
+
+
 def build_lib(verbose=False, jobs=None):
     gen_txfm()
     if not os.path.isdir(AV1CORE_INCLUDE):
         if os.path.exists(LIB):
+            print("note: no av1core headers (AV1GPU_REF or AV1CORE_INCLUDE): %s is not compiled here but used as it is, with the tables "
+                  "of headers %s" % (LIB, _built_from()[:16] or "unknown"), file=sys.stderr)
             return LIB
         raise RuntimeError("av1core headers not found at %s (set AV1GPU_REF or AV1CORE_INCLUDE)" % AV1CORE_INCLUDE)
     os.makedirs(BUILD_DIR, exist_ok=True)
+    ident = _headers_id()
+    same = _built_from() == ident
+    if not same and _built_from():
+        os.remove(os.path.join(BUILD_DIR, "headers.id"))   # until every unit is compiled from these headers
     incs = ["-I" + os.path.join(ROOT, "include"), "-I" + CSRC, "-I" + AV1CORE_INCLUDE]
     todo = []
     for src, obj, defs in UNITS:
         o = os.path.join(BUILD_DIR, obj)
-        if _newer(o, sorted(_local_deps(os.path.join(CSRC, src)))):
+        if not same or _newer(o, sorted(_local_deps(os.path.join(CSRC, src)))):
             todo.append([NVCC] + NVCC_FLAGS + defs + incs + ["-c", os.path.join(CSRC, src), "-o", o + ".tmp"])
     if todo:
         from concurrent.futures import ThreadPoolExecutor
@@ -99,6 +128,9 @@ def build_lib(verbose=False, jobs=None):
         subprocess.run([NVCC, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC"] + objs +
                        ["-o", LIB + ".tmp"], check=True)
         os.replace(LIB + ".tmp", LIB)
+    if not same:
+        with open(os.path.join(BUILD_DIR, "headers.id"), "w") as f:
+            f.write(ident + "\n")
     return LIB
 
 
