@@ -135,8 +135,8 @@ def build_lib(verbose=False, jobs=None):
 
 
 def build_oracle():
-    if not REF or not os.path.isdir(REF):
-        return None   # the GPU host has no reference checkout: the prebuilt oracle/_ref travels with the tree
+    if not REF or not os.path.isdir(os.path.join(REF, "av1core", "src")):
+        return None   # no reference checkout (or an empty folder): a prebuilt oracle/_ref, where there is one, is used
     subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "oracle"), "REF=" + REF], check=True)
     # the reference's own GPU search (measurement only: the speed bar and its decisions for BD-rate comparisons); a
     # failure here leaves the comparison out, not the build

@@ -106,3 +106,15 @@ def test_without_headers_the_library_is_named(tree, monkeypatch, capfd):
     os.remove(B.LIB)
     with pytest.raises(RuntimeError):
         B.build_lib()
+
+
+def test_oracle_needs_the_reference_sources(tree, monkeypatch):
+    """A checkout path without av1core in it (an empty folder) builds no oracle and is no error of the build."""
+    tmp, _ = tree
+    (tmp / "empty").mkdir()
+    runs = []
+    monkeypatch.setattr(B.subprocess, "run", lambda *a, **k: runs.append(a))
+    for ref in ("", str(tmp / "empty"), str(tmp / "absent")):
+        monkeypatch.setattr(B, "REF", ref)
+        assert B.build_oracle() is None
+    assert not runs
