@@ -112,6 +112,10 @@ def cpu_baseline(planes, qindex, crop=(2000, 1500), min_seconds=10.0):
     sub = [np.ascontiguousarray(planes[0][:ch, :cw]), np.ascontiguousarray(planes[1][:ch // 2, :cw // 2]),
            np.ascontiguousarray(planes[2][:ch // 2, :cw // 2])]
     threads = os.cpu_count() or 1
+    try:
+        O.lib()
+    except O.OracleMissing as ex:
+        return {"unavailable": str(ex)}
     n, t0 = 0, time.perf_counter()
     while n == 0 or time.perf_counter() - t0 < min_seconds:   # repeated searches: a sample of about 10 s
         O.encode(sub, qindex, threads=threads)
@@ -157,6 +161,11 @@ def cpu_reference(args, planes, rank):
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import oracle as O
     if rank != 0:
+        return
+    try:
+        O.lib()
+    except O.OracleMissing as ex:
+        print(json.dumps({"impl": "reference", "unavailable": str(ex)}), flush=True)
         return
     cw, ch = 2000, 1500
     crop = [np.ascontiguousarray(planes[0][:ch, :cw]), np.ascontiguousarray(planes[1][:ch // 2, :cw // 2]),

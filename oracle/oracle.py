@@ -26,11 +26,15 @@ class OrcImage(C.Structure):
 _lib = None
 
 
+class OracleMissing(RuntimeError):
+    """oracle/_ref/liboracle.so is not there (it is built from the reference's sources)."""
+
+
 def lib():
     global _lib
     if _lib is None:
         if not os.path.exists(LIB_PATH):
-            raise RuntimeError("oracle library missing: build it with `make -C oracle` (or __graft_entry__.build())")
+            raise OracleMissing("oracle library missing: build it with `make -C oracle` (or __graft_entry__.build())")
         L = C.CDLL(LIB_PATH)
         L.orc_encode.argtypes = [C.POINTER(OrcImage), C.c_int, C.POINTER(C.c_void_p)]
         L.orc_free.argtypes = [C.c_void_p]
