@@ -100,6 +100,9 @@ def build_lib(verbose=False, jobs=None):
         raise RuntimeError("av1core headers not found at %s (set AV1GPU_REF or AV1CORE_INCLUDE)" % AV1CORE_INCLUDE)
     os.makedirs(BUILD_DIR, exist_ok=True)
     ident = _headers_id()
+    kind = "checkout" if os.path.isdir(os.path.join(AV1CORE_INCLUDE, "..", "src")) else "headers only"
+    names = '-DIS_HEADERS_ID="%s, %s"' % (ident[:16], kind)
+    ident += " " + kind
     same = _built_from() == ident
     if not same and _built_from():
         os.remove(os.path.join(BUILD_DIR, "headers.id"))   # until every unit is compiled from these headers
@@ -108,7 +111,7 @@ def build_lib(verbose=False, jobs=None):
     for src, obj, defs in UNITS:
         o = os.path.join(BUILD_DIR, obj)
         if not same or _newer(o, sorted(_local_deps(os.path.join(CSRC, src)))):
-            todo.append([NVCC] + NVCC_FLAGS + defs + incs + ["-c", os.path.join(CSRC, src), "-o", o + ".tmp"])
+            todo.append([NVCC] + NVCC_FLAGS + defs + ([names] if src == "is_api.cu" else []) + incs + ["-c", os.path.join(CSRC, src), "-o", o + ".tmp"])
     if todo:
         from concurrent.futures import ThreadPoolExecutor
 

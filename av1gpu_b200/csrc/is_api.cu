@@ -536,6 +536,10 @@ void is_destroy(is_handle *h) {
 }
 
 const char *is_last_error(const is_handle *h) { return h ? h->err.c_str() : "null handle"; }
+#ifndef IS_HEADERS_ID   // (build.py names the headers)
+#define IS_HEADERS_ID "unknown, headers only"
+#endif
+const char *is_build_info(void) { return "av1core headers " IS_HEADERS_ID; }
 
 // the wavefront order (SBs by tile-local step c + 2 r) and the decode order (tiles raster, SBs raster) of an image
 static void sb_orders(const FrameDesc &F, const std::vector<int> &cs, const std::vector<int> &rs, uint32_t *order, uint32_t *dec) {

@@ -56,7 +56,7 @@ class IsTimes(C.Structure):
 
 
 # every entry point declared in include/is_api.h
-EXPORTS = ["is_create", "is_destroy", "is_last_error", "is_encode_device", "is_encode_host", "is_record_counts",
+EXPORTS = ["is_create", "is_destroy", "is_last_error", "is_build_info", "is_encode_device", "is_encode_host", "is_record_counts",
            "is_record_copy", "is_record_device", "is_times_get", "is_test_fwd_quant", "is_test_inverse",
            "is_test_predict", "is_debug_analysis", "is_debug_leaves", "is_debug_tables", "is_probe_int32", "is_set_trace", "is_get_trace",
            "is_fwd_quant_static", "is_encode_batch", "is_batch_counts", "is_batch_copy", "is_set_batch_options",
@@ -69,6 +69,11 @@ EXPORTS = ["is_create", "is_destroy", "is_last_error", "is_encode_device", "is_e
            "is_avif_mux"]
 
 _lib = None
+
+
+def build_info():
+    """Where the library's AV1 tables come from (is_build_info): "av1core headers <digest>, checkout" or ", headers only"."""
+    return load_library().is_build_info().decode()
 
 
 def load_library():
@@ -85,6 +90,8 @@ def load_library():
     L.is_destroy.restype = None
     L.is_last_error.argtypes = [vp]
     L.is_last_error.restype = C.c_char_p
+    L.is_build_info.argtypes = []
+    L.is_build_info.restype = C.c_char_p
     L.is_encode_device.argtypes = [vp, C.POINTER(IsFrame), vp]
     L.is_encode_host.argtypes = [vp, C.POINTER(IsFrame), vp]
     L.is_record_counts.argtypes = [vp, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32), C.POINTER(C.c_uint64)]

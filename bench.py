@@ -276,7 +276,7 @@ def main():
     h2d = sum(p.nbytes for p in planes)
     d2h = nb * 16 + (nb + 1) * 4 + nt * 16 + nc * 2 + sum(r.nbytes for r in out["recon"])
     if rank == 0:
-        from av1gpu_b200 import roofline
+        from av1gpu_b200 import isearch, roofline
         line = {"metric": "intra_search_mp_per_s", "value": round(value, 3), "unit": "MP/s", "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(step_ms, 3), "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic",
@@ -285,6 +285,7 @@ def main():
                 "e2e": {"value": round(e2e_value, 3), "unit": "MP/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
                 "gpu_launches": LAUNCHES_PER_STEP * args.steps,
                 "stage_ms": {k: round(v, 3) for k, v in kernel_ms.items()},
+                "library": isearch.build_info(),
                 "clocks": clk.summary()}
         line["roofline"] = roofline.report(enc, kernel_ms, mp)
         if not args.no_cpu_baseline:

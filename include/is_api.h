@@ -71,6 +71,9 @@ typedef struct is_times {
 int is_create(const is_params *p, is_handle **out);
 void is_destroy(is_handle *h);
 const char *is_last_error(const is_handle *h);
+/* What the library's AV1 tables come from: "av1core headers <digest>, checkout" (a checkout of av1core, its sources beside its
+ * headers) or "..., headers only" (headers that nothing shows to be av1core's own).  No GPU needed. */
+const char *is_build_info(void);
 
 /* Run the search on one image; stream: a cudaStream_t (NULL = the handle's own stream).  Returns after the work is
  * queued and the record sizes are known (one small device->host read). */
