@@ -57,7 +57,7 @@ class IsTimes(C.Structure):
 
 # every entry point declared in include/is_api.h
 EXPORTS = ["is_create", "is_destroy", "is_last_error", "is_build_info", "is_encode_device", "is_encode_host", "is_record_counts",
-           "is_record_copy", "is_record_device", "is_times_get", "is_test_fwd_quant", "is_test_inverse",
+           "is_record_copy", "is_record_device", "is_times_get", "is_test_fwd_quant", "is_test_eval_mixed", "is_test_inverse",
            "is_test_predict", "is_debug_analysis", "is_debug_leaves", "is_debug_tables", "is_probe_int32", "is_set_trace", "is_get_trace",
            "is_fwd_quant_static", "is_encode_batch", "is_batch_counts", "is_batch_copy", "is_set_batch_options",
            "is_autotune_batch", "is_workspace_bytes", "is_workspace_bytes_format", "is_sl_create", "is_sl_destroy", "is_sl_set_params",
@@ -98,6 +98,7 @@ def load_library():
     L.is_record_copy.argtypes = [vp, vp, vp, vp, vp, vp, vp * 3, vp]
     L.is_record_device.argtypes = [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), C.POINTER(vp)]
     L.is_times_get.argtypes = [vp, C.POINTER(IsTimes)]
+    L.is_test_eval_mixed.argtypes = [vp, C.c_int, C.c_int, C.c_int, vp, vp, C.c_int, vp, C.c_int, C.c_int, vp, vp, vp, vp, vp]
     L.is_test_fwd_quant.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, vp]
     L.is_test_inverse.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, C.c_int, vp, vp]
     L.is_test_predict.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, vp, vp]
@@ -550,6 +551,18 @@ class Encoder:
                                              coef.ctypes.data, lv.ctypes.data, D.ctypes.data, R.ctypes.data,
                                              eob.ctypes.data), "is_test_fwd_quant")
         return coef, lv, D, R, eob
+
+    def test_eval_mixed(self, form, src, pred, tx_size, tx_types, plane, qindex, ctx, bit_depth=8):
+        """Blocks of a small tx size with a tx type each through the closed loop's (form 0) or the analysis' (1) evaluation."""
+        src, pred = np.ascontiguousarray(src, np.uint16), np.ascontiguousarray(pred, np.uint16)
+        ty, cx = np.ascontiguousarray(tx_types, np.uint8), np.array(ctx, np.int32)
+        n = src.shape[0]
+        lv = np.zeros((n, src.shape[1] * src.shape[2]), np.int16)
+        D, R, eob = np.zeros(n, np.int64), np.zeros(n, np.int64), np.zeros(n, np.int32)
+        self._check(self.L.is_test_eval_mixed(self.h, form, bit_depth, n, src.ctypes.data, pred.ctypes.data, tx_size, ty.ctypes.data, plane,
+                                              qindex, cx.ctypes.data, lv.ctypes.data, D.ctypes.data, R.ctypes.data, eob.ctypes.data),
+                    "is_test_eval_mixed")
+        return lv, D, R, eob
 
     def test_inverse(self, levels, tx_size, tx_type, qindex, w, h):
         levels = np.ascontiguousarray(levels, np.int16)

@@ -259,6 +259,13 @@ int is_postfilter_from_q(int qindex, int bit_depth, av1g_frame_params *fp);
  * plane 0 luma, 1/2 chroma; ctx = (skipCtx, dcCtx, intraDir). */
 int is_test_fwd_quant(is_handle *h, int n, const int32_t *res, int tx_size, int tx_type, int plane, int qindex,
                       const int32_t ctx[3], int32_t *coef, int16_t *levels, int64_t *D, int64_t *R, int32_t *eob);
+/* The search's evaluations of the small tx sizes (4x4, 8x8, 4x8, 8x4, 4x16, 16x4), every block with a tx type of its own, so that
+ * the lanes of a warp take different ways: form 0 the closed loop's (two lanes a block), 1 the analysis' (a thread a block; it
+ * leaves the levels of 8x8, 4x16 and 16x4 blocks only, the others' are zero).  src, pred [n][H*W] samples of bit_depth 8 or 10;
+ * tx_types [n] from TX_SET_INTRA_1; outputs as is_test_fwd_quant's. */
+int is_test_eval_mixed(is_handle *h, int form, int bit_depth, int n, const uint16_t *src, const uint16_t *pred, int tx_size,
+                       const uint8_t *tx_types, int plane, int qindex, const int32_t ctx[3], int16_t *levels, int64_t *D,
+                       int64_t *R, int32_t *eob);
 /* Exact inverse transform (av1g_dequant + av1g_inv_txfm2d semantics) of n level blocks: res [n][H*W], flags [n]. */
 int is_test_inverse(is_handle *h, int n, const int16_t *levels, int tx_size, int tx_type, int qindex, int32_t *res,
                     uint32_t *flags);
