@@ -293,6 +293,21 @@ std::mutex g_upload_mu;
 bool g_uploaded[64];
 
 // the search's tables into every compilation unit's copies on device dev (once per device)
+// The neighbours base_sum and br_third add up, against av1core's tables: every neighbour's packed row has a 1 at its own place
+// only, a digit of the sum per (row, column).
+bool packed_neighbours_match() {
+    for (int cls = 0; cls < 3; cls++) {
+        const bool c2 = cls == AV1G_TX_CLASS_2D, ch = cls == AV1G_TX_CLASS_HORIZ;
+        auto place = [](int dr, int dc) -> unsigned long long { return 1ull << (2 * (dr * 5 + dc)); };   // (up to 3 of a place)
+        unsigned long long sig = 0, mag = place(0, 1) + place(1, 0);
+        for (int k = 0; k < 5; k++) sig += place(AV1G_T(Sig_Ref_Diff_Offset)[cls][k][0], AV1G_T(Sig_Ref_Diff_Offset)[cls][k][1]);
+        mag += br_third<unsigned long long>(c2, ch, place);
+        for (int k = 0; k < 3; k++) mag -= place(AV1G_T(Mag_Ref_Offset_With_Tx_Class)[cls][k][0], AV1G_T(Mag_Ref_Offset_With_Tx_Class)[cls][k][1]);
+        if (sig != base_sum<unsigned long long>(c2, ch, place) || mag) return false;
+    }
+    return true;
+}
+
 int upload_tables(int dev) {
     if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lk(g_upload_mu);
@@ -326,13 +341,7 @@ int upload_tables(int dev) {
         }
         cudaError_t e = cudaSuccess;
         // the compile-time copies of spec tables in the per-thread search must equal av1core's
-        for (int c = 0; c < 3 && e == cudaSuccess; c++) {
-            for (int k = 0; k < 5; k++)
-                if (sig_ref(c, k, 0) != AV1G_T(Sig_Ref_Diff_Offset)[c][k][0] || sig_ref(c, k, 1) != AV1G_T(Sig_Ref_Diff_Offset)[c][k][1]) e = cudaErrorInvalidValue;
-            for (int k = 0; k < 3; k++)
-                if (mag_ref(c, k, 0) != AV1G_T(Mag_Ref_Offset_With_Tx_Class)[c][k][0] || mag_ref(c, k, 1) != AV1G_T(Mag_Ref_Offset_With_Tx_Class)[c][k][1])
-                    e = cudaErrorInvalidValue;
-        }
+        if (!packed_neighbours_match()) e = cudaErrorInvalidValue;
         if (kDr23 != AV1G_T(Dr_Intra_Derivative)[23] || kDr45 != AV1G_T(Dr_Intra_Derivative)[45] || kDr67 != AV1G_T(Dr_Intra_Derivative)[67]) e = cudaErrorInvalidValue;
         for (int lw = 2; lw <= 4; lw++)
             for (int lh = 2; lw + lh <= 6; lh++)

@@ -20,12 +20,11 @@
 #include "av1g/spec_tables.h"
 #include "av1g/cdfctx.h"
 #include "txfm_gen.cuh"
+#include "is_levels.cuh"
 
 namespace is {
 
-typedef long long i64;
 constexpr i64 INF = 1LL << 60;
-constexpr int FB = 3;
 constexpr int NCDF = (int)(sizeof(av1g_cdfs) / 2);
 // plain-form knobs (reference GpConfig defaults, encoder/src/pipeline.cpp:41-76)
 constexpr int K_TOP = 4, K_RECHECK = 2, UV_K = 2;
@@ -642,9 +641,6 @@ struct ResFn {
     const P *pred;       // the prediction, W x H
     int lw;
     const int32_t *arr;  // residual array (H x W row-major) instead of src - prediction
-    __device__ __forceinline__ int operator()(int i, int j) const {
-        return arr ? arr[(i << lw) + j] : (int)src[i * sp + j] - (int)pred[(i << lw) + j];
-    }
 };
 
 // ---- lane groups: G lanes (a power of two) evaluate one task; reductions stay inside the aligned group ----
@@ -887,18 +883,15 @@ __device__ __noinline__ EvalOut grp_eval_x(int txSz, const Px *rsrc, int rsp, co
             const bool last = s == ps - 1;
             auto right = [&](const uint32_t *p, int k) -> uint32_t { return __funnelshift_r(p[0], last ? 0u : p[1], 4 * k); };   // from k columns on
             const uint32_t *a = p3 + r * ps + s, *x = p15 + r * ps + s;
-            uint32_t m = right(a, 1) + a[ps];
-            if (cls == AV1G_TX_CLASS_2D) m += right(a + ps, 1) + right(a, 2) + a[2 * ps];
-            else if (cls == AV1G_TX_CLASS_HORIZ) m += right(a, 2) + right(a, 3) + right(a, 4);
-            else m += a[2 * ps] + a[3 * ps] + a[4 * ps];
-            sums[r * ps + s] = m;
+            const bool c2 = cls == AV1G_TX_CLASS_2D, ch = cls == AV1G_TX_CLASS_HORIZ;
+            sums[r * ps + s] = base_sum<uint32_t>(c2, ch, [&](int dr, int dc) -> uint32_t { return dc ? right(a + dr * ps, dc) : a[dr * ps]; });
             const uint32_t w = x[0];
             uint32_t nz = w | w >> 1;
             nz = (nz | nz >> 2) & 0x11111111u;
             b += 256 * __popc(nz);
             if (!nz) continue;
             const uint32_t xr = right(x, 1), xd = x[ps];
-            const uint32_t xc = cls == AV1G_TX_CLASS_2D ? right(x + ps, 1) : cls == AV1G_TX_CLASS_HORIZ ? right(x, 2) : x[2 * ps];
+            const uint32_t xc = br_third<uint32_t>(c2, ch, [&](int dr, int dc) -> uint32_t { return dc ? right(x + dr * ps, dc) : x[dr * ps]; });
             const uint32_t w3 = a[0];
             uint32_t bg = (w3 & w3 >> 1) & 0x11111111u;   // levels above 2
 #pragma unroll 1

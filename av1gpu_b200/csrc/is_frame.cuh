@@ -11,6 +11,7 @@
 #pragma once
 #include <stdint.h>
 #include "av1g/decisions.h"
+#include "is_levels.cuh"
 
 namespace is {
 
@@ -104,12 +105,6 @@ struct __align__(16) FrameDesc {
     int waitIters;
     int poison;                               // fill shared memory with a pattern at kernel start (is_set_poison)
 };
-
-// a quantiser step's divisions by 64 step as multiplications: (n M) >> 32 is n / (64 step) or one less (n < 2^32)
-#ifdef __CUDACC__
-__host__ __device__
-#endif
-inline uint32_t quant_recip(int step) { return 0xFFFFFFFFu / (64u * (unsigned)step); }
 
 // error codes written to FrameDesc::err by the kernels
 constexpr int KERR_WAIT_LEAF = 2;    // a leaf dependency wait of the closed loop ran out of its iteration budget

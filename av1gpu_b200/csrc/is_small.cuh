@@ -13,11 +13,15 @@
 //   - the levels of a row lie in one word, 4 bits each (capped at 15, and at 3 for the base contexts), so the context
 //     sums of a whole row are a few shifts and additions of words instead of five bounds-checked loads a coefficient;
 //   - the scan position and the position's context offset come from one table load a coefficient.
-// quant_level, row_bits and pos_entry are also the analysis' (k_analysis_tiny, one thread a block).
+// quant_level, row_bits (is_levels.cuh) and pos_entry are also the analysis' (k_analysis_tiny, one thread a block).
 #pragma once
 #include "is_dev.cuh"
+#include "is_levels.cuh"
 
 namespace is {
+
+static_assert(TXC_2D == AV1G_TX_CLASS_2D && TXC_HORIZ == AV1G_TX_CLASS_HORIZ && EOB_STRIDE == IS_CD(coeff_base_eob, 3) &&
+              BASE_STRIDE == IS_CD(coeff_base, 3) && BR_STRIDE == IS_CD(coeff_br, 3), "is_levels.cuh");
 
 constexpr int SMALL_SIZES = 6;
 // Transform_Row_Shift of these sizes (the library checks it against av1core's table at upload)
@@ -51,81 +55,13 @@ __device__ __forceinline__ void small_tabs_stage(SmallTabs &S, const RateTabs &T
 // keeps the tasks of a warp on different banks
 template <int LW, int LH> constexpr int small_words() { return 2 * ((1 << LH) + 4) * (LW == 4 ? 2 : 1) + 1; }
 
-template <int LW> using PackedRow = typename std::conditional<LW == 4, unsigned long long, uint32_t>::type;   // 4 bits a column
-
-// bits of the coefficients of row rr of a tx block of 1 << LW columns whose levels are packed 4 bits each: a0 .. a4 the rows
-// rr .. rr + 4 capped at 3, b0 .. b2 the rows rr .. rr + 2 capped at 15 (a3, a4 and b2 are used by the vertical class only).
-// Every sign counts one bit (the caller corrects the DC's).  tab: scan position | context offset << 8 of the row's
-// positions; level(j): the signed level of column j.
-template <int LW, int LH, typename Level>
-__device__ __forceinline__ int row_bits(int rr, PackedRow<LW> a0, PackedRow<LW> a1, PackedRow<LW> a2, PackedRow<LW> a3, PackedRow<LW> a4,
-                                        PackedRow<LW> b0, PackedRow<LW> b1, PackedRow<LW> b2, int cls, int eob, const uint16_t *tab,
-                                        const uint16_t *cBase, const uint16_t *cEob, const uint16_t *cBr, const Level &level) {
-    typedef PackedRow<LW> Row;
-    constexpr int W = 1 << LW, N = 1 << (LW + LH);
-    int b = 0;
-    const bool c2 = cls == AV1G_TX_CLASS_2D, ch = cls == AV1G_TX_CLASS_HORIZ;
-    // the base contexts' neighbours (at most 5 of at most 3: 4 bits a sum), and the third neighbour of the ranges' contexts,
-    // beside (0, 1) and (1, 0)
-    const Row m = (a0 >> 4) + a1 + (c2 ? (a1 >> 4) + (a0 >> 8) + a2 : ch ? (a0 >> 8) + (a0 >> 12) + (a0 >> 16) : a2 + a3 + a4);
-    const Row x2 = c2 ? b1 >> 4 : ch ? b0 >> 8 : b2;
-    // base symbols of the row, without branches: a coefficient past the end of block costs nothing, the last one takes
-    // the end-of-block table
-    Row big = 0;
-#pragma unroll
-    for (int j = 0; j < W; j++) {
-        const int t = tab[j], c = t & 0xFF, l3 = (int)(a0 >> (4 * j)) & 3;
-        int ctx = min(((int)(m >> (4 * j) & 15) + 1) >> 1, 4) + (t >> 8);
-        if (j == 0) ctx = rr == 0 && cls == AV1G_TX_CLASS_2D ? 0 : ctx;
-        const int ectx = c == 0 ? 0 : c <= N / 8 ? 1 : c <= N / 4 ? 2 : 3;
-        // (a valid entry for every coefficient: the last one's level is at least 1)
-        const int bits = *(c == eob - 1 ? cEob + ectx * IS_CD(coeff_base_eob, 3) + l3 - 1 : cBase + ctx * IS_CD(coeff_base, 3) + l3);
-        b += (c < eob ? bits : 0) + (l3 ? 256 : 0);
-        big |= (Row)(l3 > 2 ? 1 : 0) << (4 * j);
-    }
-    // the ranges and remainders of the levels above 2, one after the other
-#pragma unroll 1
-    for (; big; big &= big - 1) {
-        const int sh = LW == 4 ? __ffsll((long long)big) - 1 : __ffs((int)big) - 1, j = sh >> 2;
-        const int l = (int)(b0 >> sh) & 15, right = (int)((b0 >> sh) >> 4) & 15;
-        int mg = right + ((int)(b1 >> sh) & 15) + ((int)(x2 >> sh) & 15);
-        mg = min((mg + 1) >> 1, 6);
-        const int near = cls == AV1G_TX_CLASS_2D ? (rr < 2 && j < 2) : cls == AV1G_TX_CLASS_HORIZ ? j == 0 : rr == 0;
-        const uint16_t *cr = cBr + ((rr | j) == 0 ? mg : near ? mg + 7 : mg + 14) * IS_CD(coeff_br, 3);
-        const int rem = l - 3, full = (rem * 11) >> 5;   // rem / 3: at most 4 symbols
-        b += full * cr[3];
-        if (full < 4) b += cr[rem - 3 * full];
-        if (l == 15) {
-            const int v = abs(level(j));
-            if (v > 14) b += (2 * (31 - __clz(v - 14)) + 1) * 256;
-        }
-    }
-    return b;
-}
-
-// level of a coefficient, its distance from the dequantised value and its packed forms (tx sizes of dequantisation
-// denominator 1); no branch: the coefficients of a row are independent chains.  M: quant_recip(step)
-template <int BD>
-__device__ __forceinline__ int quant_level(int v, int step, uint32_t M, i64 &dist) {
-    const int a = abs(v), St = step << FB;
-    const uint32_t n = (uint32_t)(8 * a + 3 * St), d = (uint32_t)(8 * St);
-    uint32_t u = __umulhi(n, M);   // n / d or one less
-    u += n - u * d >= d;
-    const int l = a * 32 >= 21 * St ? min((int)u, 16383) : 0;
-    // |dequantised|: 24 bits, clamped to 2^(7 + BD) below and one less above zero
-    const int dq = min((l * step) & 0xFFFFFF, (1 << (7 + BD)) - (v >= 0 ? 1 : 0));
-    const int df = a - dq * (1 << FB);
-    dist += (i64)df * df;
-    return v < 0 ? -l : l;
-}
-
 // One evaluation by lanes g = 0, 1 of a pair (all lanes of the warp call it together): src and pred are W x H in shared
 // memory, rows are small_words() words of scratch and q the W x H levels of the task.  dcM / acM: floor(2^32 / (64 step)).
 template <int BD, int LW, int LH, typename Px>
 __device__ __forceinline__ EvalOut small_eval(int si, const Px *src, const Px *pred, int txType, int plane, int skipCtx, int dcCtx, int intraDir,
                                               int dcQ, int acQ, uint32_t dcM, uint32_t acM, const uint16_t *C, const SmallTabs &S,
                                               int32_t *buf, uint32_t *rows, int16_t *q, int g) {
-    constexpr int W = 1 << LW, H = 1 << LH, N = W * H, CW = W / 2, RH = H / 2;
+    constexpr int W = 1 << LW, H = 1 << LH, CW = W / 2, RH = H / 2;
     typedef PackedRow<LW> Row;
     const int txSz = LW == LH ? (LW == 2 ? AV1G_TX_4X4 : AV1G_TX_8X8) : LW == 2 ? (LH == 3 ? AV1G_TX_4X8 : AV1G_TX_4X16)
                    : LW == 3 ? AV1G_TX_8X4 : AV1G_TX_16X4;

@@ -28,19 +28,7 @@
 
 namespace is {
 
-// Spec constants fixed at compile time (the library checks them against av1core's tables at upload): Sig_Ref_Diff_Offset and
-// Mag_Ref_Offset_With_Tx_Class (spec 8.3.2), which the row and column shifts of packed levels (row_bits, grp_eval_x) spell
-// out, and Dr_Intra_Derivative at 23, 45, 67 degrees.
-// (row, column) offset d of neighbour k for tx class c (0 2D, 1 HORIZ, 2 VERT)
-__host__ __device__ constexpr int sig_ref(int c, int k, int d) {
-    return k == 0 ? (d == 0 ? 0 : 1) : k == 1 ? (d == 0 ? 1 : 0)
-         : c == 0 ? (k == 2 ? 1 : k == 3 ? (d == 0 ? 0 : 2) : (d == 0 ? 2 : 0))
-         : c == 1 ? (d == 0 ? 0 : k) : (d == 0 ? k : 0);
-}
-__host__ __device__ constexpr int mag_ref(int c, int k, int d) {
-    return k == 0 ? (d == 0 ? 0 : 1) : k == 1 ? (d == 0 ? 1 : 0)
-         : c == 0 ? 1 : c == 1 ? (d == 0 ? 0 : 2) : (d == 0 ? 2 : 0);
-}
+// Dr_Intra_Derivative at 23, 45 and 67 degrees, fixed at compile time (the library checks them against av1core's table at upload)
 constexpr int kDr23 = 151, kDr45 = 64, kDr67 = 27;
 
 constexpr int TINY_THREADS = 256;
