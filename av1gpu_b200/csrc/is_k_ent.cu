@@ -22,6 +22,7 @@
 // A symbol is one 32-bit word: kind (adaptive / equiprobable bit / split-or-horizontal / split-or-vertical), alphabet
 // size, value and the CDF's offset inside av1g_cdfs.
 #include "is_units.cuh"
+#include "is_range.cuh"
 #include "is_api.h"
 #include <algorithm>
 #include <cstring>
@@ -602,14 +603,6 @@ __global__ void k_ent_emit_txb(EntArgs A) {
 }
 
 // ---- CDF adaptation: the symbols' interval bounds ----
-// A coder step of symbol s of an alphabet of nm1 + 1 symbols with bounds fl / fh (32768 x the probability of the
-// symbols after s - 1 / after s): the upper half holds fl's bits from 6 on (the coder reads no lower ones; bit 15 set: fl
-// is the whole range, symbol 0) and nm1 - s below them, the lower half fh
-__device__ __forceinline__ uint32_t step_hi(uint32_t fl, int below) { return (fl & 0xFFC0u) | (uint32_t)below; }
-__device__ __forceinline__ uint32_t pack_step(uint32_t fl, uint32_t fh, int s, int nm1) { return (step_hi(fl, nm1 - s) << 16) | fh; }
-constexpr uint32_t STEP_FIRST = 1u << 31;
-__device__ __forceinline__ uint32_t step_ev(uint32_t e) { return (e >> 14) & 0xFCu; }   // 4 (nm1 - s)
-
 // the CDFs the symbols use, numbered: CDF i starts at entry g_cdfOff[i] of av1g_cdfs and has g_cdfN[i] symbols;
 // g_cdfId[offset / 3] is its number (distinct CDFs start at least 3 entries apart)
 constexpr int NID_MAX = 1536;
@@ -805,18 +798,6 @@ __global__ void __launch_bounds__(CS_T) k_ent_scatter(EntArgs A) {
     }
 }
 
-// The CDFs in the inverse form of the bounds, a = 32768 - c: symbol s has fl = a[s - 1] (32768 for s = 0) and fh = a[s] (0
-// for the last); spec 8.2.6's adaptation moves entries before s up by (32768 - a) >> rate and the others down by
-// a >> rate, which is a += (T - a) >> rate with T = 32768 or 2^rate - 1 (the arithmetic shift rounds down).
-// A lane holds one entry a: 4 lanes walk a CDF of up to 4 symbols, 16 a larger one.  The lane of entry s leaves the
-// step's lower half, that of entry s - 1 the upper one (the last lane for s = 0), so a symbol costs no exchange between
-// lanes.  One lane with the three entries of a small CDF, the bounds selected and packed, took 100 cycles a symbol.
-__device__ __forceinline__ void adapt_entry(int &a, int j, int s, int nm1, int last, int rate, uint16_t *at) {
-    const int up = s > j;
-    if (j == s) at[0] = (uint16_t)a;
-    if (s ? j == s - 1 : j == last) at[1] = (uint16_t)step_hi(s ? (uint32_t)a : 32768u, nm1 - s);
-    a += ((up ? 32768 : (1 << rate) - 1) - a) >> rate;
-}
 __global__ void __launch_bounds__(32) k_ent_adapt(EntArgs A, int smallWarps, int nSmall, int nLarge, int warpsPerTile) {
     if (A.status->error) return;
     const uint32_t t = blockIdx.x / warpsPerTile;
@@ -919,30 +900,6 @@ __global__ void __launch_bounds__(32) k_ent_adapt(EntArgs A, int smallWarps, int
 //                 into 16-bit digits (held in 32 bits) at their places, k_rg_carry carries them through.
 constexpr int RG_CH = 1024;            // steps per chunk (nominal: a chunk starts at the first step from there that is
                                        // not a STEP_FIRST; a stretch without one belongs to the chunk before)
-constexpr int RG_STATES = 128;
-
-// one range step in a form with a short dependent chain.  The range is held as the float bits of the unnormalised
-// range: its mantissa is the normalised one, so the renormalisation is an addition (the magic-number conversion of the
-// 16-bit sum), and (r >> 8) in bits 16-23 gives ((r >> 8) p) >> 1 as the upper word of one product with p << 15.
-struct RangeStep {
-    uint32_t mu, mv, keep, k;          // p of fl and fh << 15 (0 for fl of a STEP_FIRST); 0xFFFF for a STEP_FIRST; the rest
-};
-__device__ __forceinline__ RangeStep range_step(uint32_t e) {
-    const bool first = e & STEP_FIRST;
-    RangeStep s;
-    s.mu = first ? 0u : (e & 0xFFC00000u) >> 7;
-    s.mv = (e & 0xFFC0u) << 9;
-    s.keep = first ? 0xFFFFu : 0u;
-    s.k = 0x4B000000u + (first ? 0u - step_ev(e) : 4u);
-    return s;
-}
-__device__ __forceinline__ uint32_t range_bits(uint32_t r) { return __float_as_uint((float)r); }
-__device__ __forceinline__ uint32_t range_of(uint32_t b) { return ((b >> 8) & 0x7FFFu) | 0x8000u; }   // the normalised range
-__device__ __forceinline__ uint32_t range_next(uint32_t b, const RangeStep &s) {   // float bits of u - v
-    const uint32_t r8 = (b & 0x7F0000u) | 0x800000u;
-    const uint32_t rn = (__umulhi(r8, s.mu) + s.k) - __umulhi(r8, s.mv) + (range_of(b) & s.keep);
-    return __float_as_uint(__uint_as_float(rn) - 8388608.0f);
-}
 
 // chunk slots: tile t's chunk k is slot symBegin[t] / RG_CH + t + k
 __device__ __forceinline__ uint64_t rg_slot0(const EntArgs &A, uint32_t t) { return A.symBegin[t] / RG_CH + t; }
@@ -1085,11 +1042,8 @@ __global__ void __launch_bounds__(32) k_rg_walk(EntArgs A) {
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     if (j0 + i >= n) break;
-                    const uint32_t e = now[i], r = range_of(b);
-                    const uint32_t u = (e & STEP_FIRST) ? r : (((r >> 8) * (e >> 22)) >> 1) + step_ev(e) + 4u;
-                    b = range_next(b, range_step(e));
-                    const uint32_t d = 15u + 127u - (b >> 23);
-                    p[j0 + i] = (r - u) | (d << 16);
+                    uint32_t d;
+                    p[j0 + i] = range_term(now[i], b, d);
                     bits += d;
                 }
             }
@@ -1099,16 +1053,6 @@ __global__ void __launch_bounds__(32) k_rg_walk(EntArgs A) {
     }
 }
 
-// bytes of a tile whose steps shifted c bits out: the whole bytes sent while coding (the first after 9 bits), then the
-// flush, which sends what is left of c + 1 bits
-__device__ __forceinline__ uint32_t rg_bytes(uint64_t c) {
-    const uint64_t n0 = c >= 9 ? (c - 9) / 8 + 1 : 0;
-    const int s = (int)((long long)c - 9 - 8 * (long long)n0) + 10;
-    return (uint32_t)(n0 + (s + 7) / 8);
-}
-// a tile's digits: bit i of the payload (0 the first byte's top bit) is bit i + 16 from the top of the digits; a term of
-// 16 bits after c shifted bits starts at bit c + 15
-__device__ __forceinline__ uint64_t rg_digits(uint32_t bytes) { return (bytes + 1) / 2 + 4; }
 __device__ __forceinline__ uint32_t *rg_digit0(const EntArgs &A, uint32_t t) { return A.rgDigit + A.symBegin[t] + 16 * (uint64_t)t; }
 
 // per tile: the bits before each chunk, the payload's size, the digits cleared
@@ -1170,7 +1114,7 @@ __global__ void __launch_bounds__(128) k_rg_bits(EntArgs A) {
             const uint64_t q = c + inc - d + 15;
             const uint32_t a = (uint32_t)q & 15;
             // the terms that start in the same digit are neighbours: summed first, then one addition per digit
-            uint32_t hi = x >> a, lo = (x << (16 - a)) & 0xFFFFu;
+            uint32_t hi = digit_hi(x, a), lo = digit_lo(x, a);
             const uint32_t base = (uint32_t)(q >> 4) - (uint32_t)((c + 15) >> 4);
             const uint32_t same = __match_any_sync(0xffffffffu, base);
             hi = __reduce_add_sync(same, hi);
@@ -1184,8 +1128,8 @@ __global__ void __launch_bounds__(128) k_rg_bits(EntArgs A) {
         if (lane == 0 && end == A.symBegin[t + 1]) {   // the flush rounds up by 0x3FFF after the last step
             const uint64_t q = c + 15;
             const uint32_t a = (uint32_t)q & 15;
-            atomicAdd(dig + (q >> 4), 0x3FFFu >> a);
-            atomicAdd(dig + (q >> 4) + 1, (0x3FFFu << (16 - a)) & 0xFFFFu);
+            atomicAdd(dig + (q >> 4), digit_hi(RG_ROUND, a));
+            atomicAdd(dig + (q >> 4) + 1, digit_lo(RG_ROUND, a));
         }
     }
 }
@@ -1207,25 +1151,22 @@ __global__ void __launch_bounds__(SCAN_T) k_rg_carry(EntArgs A) {
         uint32_t v = 0;
         if (i < nd) {
             const uint64_t m = nd - 1 - i;
-            const uint32_t d0 = d[m], d1 = m + 1 < nd ? d[m + 1] : 0u, d2 = m + 2 < nd ? d[m + 2] : 0u;
-            const uint32_t n0 = (d0 & 0xFFFFu) + (d1 >> 16), n1 = (d1 & 0xFFFFu) + (d2 >> 16);
-            v = (n0 & 0xFFFFu) + (n1 >> 16);
+            v = digit_sum(d[m], m + 1 < nd ? d[m + 1] : 0u, m + 2 < nd ? d[m + 2] : 0u);
         }
         const uint32_t gen = __ballot_sync(0xffffffffu, v > 0xFFFFu), prop = __ballot_sync(0xffffffffu, v == 0xFFFFu);
-        // carries of a + b: a = gen | prop, b = gen; a warp generates without a carry in, propagates with one
-        const uint32_t a = gen | prop;
-        const uint64_t w0 = (uint64_t)a + gen, w1 = w0 + 1;
-        if (lane == 0) { gw[warp] = (uint32_t)(w0 >> 32); pw[warp] = (uint32_t)(w1 >> 32); }
+        if (lane == 0) {   // a warp generates without a carry in, propagates with one
+            gw[warp] = carry_out(gen, gen | prop, 0);
+            pw[warp] = carry_out(gen, gen | prop, 1);
+        }
         __syncthreads();
         if (warp == 0) {
             const uint32_t G = __ballot_sync(0xffffffffu, gw[lane] != 0), P = __ballot_sync(0xffffffffu, pw[lane] != 0);
-            const uint64_t sum = (uint64_t)P + G + cin;
-            if (lane == 0) cw = (uint32_t)sum ^ P ^ G;   // carry into each warp
-            cin = (uint32_t)(sum >> 32);
+            if (lane == 0) cw = carries_in(G, P, cin);   // carry into each warp
+            cin = carry_out(G, P, cin);
         }
         __syncthreads();
         const uint32_t wc = (cw >> warp) & 1;
-        const uint32_t cr = ((uint32_t)(w0 + wc) ^ a ^ gen) >> lane & 1;
+        const uint32_t cr = carries_in(gen, gen | prop, wc) >> lane & 1;
         v = (v + cr) & 0xFFFFu;
         if (i < nd) {
             const uint64_t m = nd - 1 - i;
@@ -1233,11 +1174,7 @@ __global__ void __launch_bounds__(SCAN_T) k_rg_carry(EntArgs A) {
 #pragma unroll
                 for (int z = 0; z < 2; z++) {
                     const uint64_t at = 2 * (m - 1) + z;   // byte of the payload, bits 8 at .. 8 at + 7
-                    uint32_t x = (z ? v : v >> 8) & 0xFFu;
-                    const long long last = (long long)c - 8 * (long long)at;   // the flush sets bit c and clears those after it
-                    if (last < 0) x = 0;
-                    else if (last < 8) x = (x & (0xFF00u >> last)) | (0x80u >> last);
-                    if (at < bytes) out[at] = (uint8_t)x;
+                    if (at < bytes) out[at] = payload_byte((z ? v : v >> 8) & 0xFFu, c, at);
                 }
             }
         }
@@ -1390,6 +1327,30 @@ struct Plan {
 
 size_t al(size_t v) { return (v + 255) & ~(size_t)255; }
 
+// the coder's part of a plan (P.cap symbols, P.nTiles tiles) after the first o bytes
+void plan_code(Plan &P, size_t &o) {
+    auto take = [&](size_t bytes) { const size_t at = o; o = al(o + bytes); return at; };
+    P.oSyms = take(4ull * P.cap);
+    P.oBegin = take(8ull * (P.nTiles + 1));
+    const uint64_t outN = 2 * P.cap + 16ull * P.nTiles;   // at most 15 bits a symbol, and the flush
+    const uint64_t slots = P.cap / RG_CH + P.nTiles + 1;
+    P.oRgStart = take(8 * slots);
+    P.oRgBit0 = take(8 * slots);
+    P.oRgBits = take(4 * slots);
+    P.oRgFirst = take(slots);
+    P.oRgLast = take(slots);
+    P.oRgMap = take((uint64_t)RG_STATES * slots);
+    P.oRgDigit = take(4 * (P.cap + 16ull * P.nTiles));
+    P.oTileBits = take(8ull * P.nTiles);
+    P.csPitch = ((uint32_t)cdf_list().off.size() + 7) & ~7u;
+    P.oCsTab = take(4ull * P.csPitch * (P.cap / CS_B + P.nTiles + 1));
+    P.oCsStart = take(4ull * P.csPitch * P.nTiles);
+    P.oCsLen = take(4ull * P.csPitch * P.nTiles);
+    P.oTileBytes = take(4ull * P.nTiles);
+    P.oResult = take(sizeof(is_ent_status) + 8ull * (P.nTiles + 1));
+    P.oOut = take(outN);
+}
+
 int plan(const is_ent_frame *frames, int n, uint64_t cap, Plan &P, std::string *err) {
     if (n < 1 || !frames) { if (err) *err = "no frames"; return IS_ERR_INVALID; }
     P.fr.resize(n);
@@ -1458,27 +1419,58 @@ int plan(const is_ent_frame *frames, int n, uint64_t cap, Plan &P, std::string *
     P.oHeadW = take(4ull * HEAD_WORDS * P.nB);
     P.oPartB = take(4ull * (npB + 1));
     P.oPartT = take(4ull * (npT + 1));
-    P.oSyms = take(4ull * P.cap);
-    P.oBegin = take(8ull * (P.nTiles + 1));
-    const uint64_t outN = 2 * P.cap + 16ull * P.nTiles;   // at most 15 bits a symbol, and the flush
-    const uint64_t slots = P.cap / RG_CH + P.nTiles + 1;
-    P.oRgStart = take(8 * slots);
-    P.oRgBit0 = take(8 * slots);
-    P.oRgBits = take(4 * slots);
-    P.oRgFirst = take(slots);
-    P.oRgLast = take(slots);
-    P.oRgMap = take((uint64_t)RG_STATES * slots);
-    P.oRgDigit = take(4 * (P.cap + 16ull * P.nTiles));
-    P.oTileBits = take(8ull * P.nTiles);
-    P.csPitch = ((uint32_t)cdf_list().off.size() + 7) & ~7u;
-    P.oCsTab = take(4ull * P.csPitch * (P.cap / CS_B + P.nTiles + 1));
-    P.oCsStart = take(4ull * P.csPitch * P.nTiles);
-    P.oCsLen = take(4ull * P.csPitch * P.nTiles);
-    P.oTileBytes = take(4ull * P.nTiles);
-    P.oResult = take(sizeof(is_ent_status) + 8ull * (P.nTiles + 1));
-    P.oOut = take(outN);
+    plan_code(P, o);
     P.bytes = o;
     return IS_OK;
+}
+
+// the coder's buffers of a plan in the scratch
+void code_buffers(EntArgs &A, const Plan &P, uint8_t *S) {
+    A.nTiles = P.nTiles;
+    A.syms = (uint32_t *)(S + P.oSyms);
+    A.cap = P.cap;
+    A.symBegin = (uint64_t *)(S + P.oBegin);
+    A.rgStart = (uint64_t *)(S + P.oRgStart);
+    A.rgBit0 = (uint64_t *)(S + P.oRgBit0);
+    A.rgBits = (uint32_t *)(S + P.oRgBits);
+    A.rgFirst = S + P.oRgFirst;
+    A.rgLast = S + P.oRgLast;
+    A.rgMap = S + P.oRgMap;
+    A.rgDigit = (uint32_t *)(S + P.oRgDigit);
+    A.tileBits = (uint64_t *)(S + P.oTileBits);
+    A.csTab = (uint32_t *)(S + P.oCsTab);
+    A.csStart = (uint32_t *)(S + P.oCsStart);
+    A.csLen = (uint32_t *)(S + P.oCsLen);
+    A.csPitch = P.csPitch;
+    A.tileBytes = (uint32_t *)(S + P.oTileBytes);
+    A.status = (is_ent_status *)(S + P.oResult);
+    A.tileOff = (uint64_t *)(S + P.oResult + sizeof(is_ent_status));
+    A.out = S + P.oOut;
+}
+
+// The coding of symbol words in A.syms (A.symBegin: the tiles' parts) into the payloads: CDF adaptation, then the range coder.
+// The counts of batches and chunks are known on the device only: grids for the symbol capacity, at most a few waves of the GPU.
+constexpr unsigned GPU_SMS = 148;
+void code_launch(const EntArgs &A, cudaStream_t s) {
+    auto grid = [](uint64_t n, int t) { return (unsigned)std::max<uint64_t>(1, (n + t - 1) / t); };
+    const uint64_t batches = A.cap / CS_B + A.nTiles;
+    const CdfList &L = cdf_list();
+    const int nSmall = (int)std::count_if(L.n.begin(), L.n.end(), [](uint8_t v) { return v <= 4; }), nLarge = (int)L.n.size() - nSmall;
+    const int sw = (nSmall + 7) / 8, wpt = sw + (nLarge + 1) / 2;
+    k_ent_count<<<(unsigned)std::min<uint64_t>(batches, 4 * GPU_SMS), CS_T, 0, s>>>(A);
+    k_ent_place<<<A.nTiles, SCAN_T, 0, s>>>(A);
+    k_ent_scatter<<<(unsigned)std::min<uint64_t>(batches, 2 * GPU_SMS), CS_T, sizeof(CsSmem), s>>>(A);
+    k_ent_adapt<<<(unsigned)wpt * A.nTiles, 32, 0, s>>>(A, sw, nSmall, nLarge, wpt);
+    const uint64_t slots = A.cap / RG_CH + A.nTiles;
+    auto wave = [&](uint64_t perCta, unsigned most) { return (unsigned)std::min<uint64_t>(most, grid(slots, (int)perCta)); };
+    k_rg_starts<<<wave(64, 8 * GPU_SMS), 64, 0, s>>>(A);
+    k_rg_map<<<wave(1, 16 * GPU_SMS), RG_STATES, 0, s>>>(A);
+    k_rg_chain<<<A.nTiles, 32, 0, s>>>(A);
+    k_rg_walk<<<wave(32, 16 * GPU_SMS), 32, 0, s>>>(A);
+    k_rg_offs<<<A.nTiles, SCAN_T, 0, s>>>(A);
+    k_ent_offsets<<<1, SCAN_T, 0, s>>>(A);
+    k_rg_bits<<<wave(4, 16 * GPU_SMS), 128, 0, s>>>(A);
+    k_rg_carry<<<A.nTiles, SCAN_T, 0, s>>>(A);
 }
 
 }  // namespace
@@ -1506,7 +1498,7 @@ int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, s
     A.nF = n;
     uint32_t *bases = (uint32_t *)(S + P.oBases);
     A.fBlock = bases; A.fTxb = bases + (n + 1); A.fSb = bases + 2 * (n + 1); A.fTile = bases + 3 * (n + 1);
-    A.nB = P.nB; A.nT = P.nT; A.nSb = P.nSb; A.nTiles = P.nTiles;
+    A.nB = P.nB; A.nT = P.nT; A.nSb = P.nSb;
     A.miSize = S + P.oMi; A.yMode = A.miSize + P.nMi; A.skip = A.yMode + P.nMi;
     A.cul = S + P.oCtx; A.dcc = A.cul + P.nCtx;
     A.txbType = S + P.oType;
@@ -1516,25 +1508,7 @@ int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, s
     A.txbCnt = (uint32_t *)(S + P.oTxbCnt);
     A.headCnt = (uint32_t *)(S + P.oHeadCnt);
     A.headW = (uint32_t *)(S + P.oHeadW);
-    A.syms = (uint32_t *)(S + P.oSyms);
-    A.cap = P.cap;
-    A.symBegin = (uint64_t *)(S + P.oBegin);
-    A.rgStart = (uint64_t *)(S + P.oRgStart);
-    A.rgBit0 = (uint64_t *)(S + P.oRgBit0);
-    A.rgBits = (uint32_t *)(S + P.oRgBits);
-    A.rgFirst = S + P.oRgFirst;
-    A.rgLast = S + P.oRgLast;
-    A.rgMap = S + P.oRgMap;
-    A.rgDigit = (uint32_t *)(S + P.oRgDigit);
-    A.tileBits = (uint64_t *)(S + P.oTileBits);
-    A.csTab = (uint32_t *)(S + P.oCsTab);
-    A.csStart = (uint32_t *)(S + P.oCsStart);
-    A.csLen = (uint32_t *)(S + P.oCsLen);
-    A.csPitch = P.csPitch;
-    A.tileBytes = (uint32_t *)(S + P.oTileBytes);
-    A.status = (is_ent_status *)(S + P.oResult);
-    A.tileOff = (uint64_t *)(S + P.oResult + sizeof(is_ent_status));
-    A.out = S + P.oOut;
+    code_buffers(A, P, S);
     std::vector<uint32_t> hb;
     hb.insert(hb.end(), P.fBlock.begin(), P.fBlock.end());
     hb.insert(hb.end(), P.fTxb.begin(), P.fTxb.end());
@@ -1565,26 +1539,7 @@ int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, s
         k_ent_tiles<<<grid(P.nTiles, 128), 128, 0, s>>>(A);
         k_ent_emit_head<<<grid(P.nB, 256), 256, 0, s>>>(A);
         if (P.nT) k_ent_emit_txb<<<grid(P.nT, 128), 128, 0, s>>>(A);
-        // the batches' and chunks' counts are known on the device only: grids for the symbol capacity, at most a few waves
-        // of the GPU
-        const uint64_t batches = P.cap / CS_B + P.nTiles;
-        const CdfList &L = cdf_list();
-        const int nSmall = (int)std::count_if(L.n.begin(), L.n.end(), [](uint8_t v) { return v <= 4; }), nLarge = (int)L.n.size() - nSmall;
-        const int sw = (nSmall + 7) / 8, wpt = sw + (nLarge + 1) / 2;
-        k_ent_count<<<(unsigned)std::min<uint64_t>(batches, 592), CS_T, 0, s>>>(A);
-        k_ent_place<<<P.nTiles, SCAN_T, 0, s>>>(A);
-        k_ent_scatter<<<(unsigned)std::min<uint64_t>(batches, 296), CS_T, sizeof(CsSmem), s>>>(A);
-        k_ent_adapt<<<(unsigned)wpt * P.nTiles, 32, 0, s>>>(A, sw, nSmall, nLarge, wpt);
-        const uint64_t slots = P.cap / RG_CH + P.nTiles;
-        auto wave = [&](uint64_t perCta, unsigned most) { return (unsigned)std::min<uint64_t>(most, grid(slots, (int)perCta)); };
-        k_rg_starts<<<wave(64, 1184), 64, 0, s>>>(A);
-        k_rg_map<<<wave(1, 2368), RG_STATES, 0, s>>>(A);
-        k_rg_chain<<<P.nTiles, 32, 0, s>>>(A);
-        k_rg_walk<<<wave(32, 2368), 32, 0, s>>>(A);
-        k_rg_offs<<<P.nTiles, SCAN_T, 0, s>>>(A);
-        k_ent_offsets<<<1, SCAN_T, 0, s>>>(A);
-        k_rg_bits<<<wave(4, 2368), 128, 0, s>>>(A);
-        k_rg_carry<<<P.nTiles, SCAN_T, 0, s>>>(A);
+        code_launch(A, s);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -1599,6 +1554,69 @@ int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, s
     if (frameTile0)
         for (int i = 0; i <= n; i++) frameTile0[i] = P.fTile[i];
     return IS_OK;
+}
+
+// kernel test: the coder alone on symbol words of the caller's (host arrays; sym_word's layout), one CDF context for all tiles
+int ent_test_code(int nTiles, const uint64_t *begin, const uint32_t *words, int qctx, uint8_t *out, uint64_t cap, uint64_t *off, std::string *err) {
+    auto bad = [&](const char *why) { if (err) *err = why; return IS_ERR_INVALID; };
+    const CdfList &L = cdf_list();
+    if (nTiles < 1 || nTiles > 4096 || begin[0] != 0) return bad("tiles");
+    for (int t = 0; t < nTiles; t++)
+        if (begin[t + 1] <= begin[t] || begin[t + 1] > (1u << 28)) return bad("a tile's symbols");
+    const uint64_t n = begin[nTiles];
+    for (uint64_t i = 0; i < n; i++) {
+        const uint32_t w = words[i], kind = w & 3, nm1 = (w >> 2) & 15, s = (w >> 6) & 15, o = w >> 16;
+        if (kind == SYM_BIT) { if (nm1 != 1 || s > 1) return bad("a bit"); continue; }
+        if (o >= (uint32_t)NCDF || L.off[L.id[o / 3]] != o) return bad("a CDF offset");
+        const uint32_t N = L.n[L.id[o / 3]];
+        if (kind == SYM_ADAPT ? nm1 + 1 != N || s >= N : N != 10 || nm1 != 1 || s > 1) return bad("a symbol");
+    }
+    Plan P;
+    P.nTiles = (uint32_t)nTiles;
+    P.cap = n;
+    size_t o = 0, oFr = o, oTile = al(sizeof(EntFrameD));
+    o = oTile + al(8);
+    plan_code(P, o);
+    uint8_t *S = nullptr;
+    cudaError_t e = cudaMalloc(&S, o);
+    if (e != cudaSuccess) { if (err) *err = "scratch"; return IS_ERR_OOM; }
+    EntArgs A;
+    memset(&A, 0, sizeof A);
+    EntFrameD F;
+    memset(&F, 0, sizeof F);
+    F.qctx = qctx & 3;
+    const uint32_t fTile[2] = {0, (uint32_t)nTiles};
+    A.fr = (const EntFrameD *)(S + oFr);
+    A.fTile = (const uint32_t *)(S + oTile);
+    A.nF = 1;
+    code_buffers(A, P, S);
+    if (e == cudaSuccess) e = cudaMemcpy(S + oFr, &F, sizeof F, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(S + oTile, fTile, 8, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(A.status, 0, sizeof(is_ent_status));
+    if (e == cudaSuccess) e = cudaMemcpy(A.symBegin, begin, 8 * (nTiles + 1), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(A.syms, words, 4 * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) { code_launch(A, 0); e = cudaGetLastError(); }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    is_ent_status st;
+    if (e == cudaSuccess) e = cudaMemcpy(&st, A.status, sizeof st, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(off, A.tileOff, 8 * (nTiles + 1), cudaMemcpyDeviceToHost);
+    int rc = IS_OK;
+    if (e == cudaSuccess && (st.error || off[nTiles] > cap)) { if (err) *err = "coder status"; rc = IS_ERR_TOO_LARGE; }
+    if (e == cudaSuccess && !rc) e = cudaMemcpy(out, A.out, off[nTiles], cudaMemcpyDeviceToHost);
+    cudaFree(S);
+    if (e != cudaSuccess) { if (err) *err = cudaGetErrorString(e); return IS_ERR_CUDA; }
+    return rc;
+}
+// the CDFs of a q-context at the start of a tile (av1g_cdfs entries), and where each begins and its symbols; their number
+int ent_test_cdfs(int qctx, uint16_t *cdf, size_t cap, uint16_t *off, uint8_t *n) {
+    const int qrep[4] = {20, 60, 120, 255};
+    av1g_cdfs c;
+    av1g_cdfs_init(&c, qrep[qctx & 3]);
+    if (cdf) memcpy(cdf, &c, std::min(cap, (size_t)NCDF) * 2);
+    const CdfList &L = cdf_list();
+    if (off) memcpy(off, L.off.data(), L.off.size() * 2);
+    if (n) memcpy(n, L.n.data(), L.n.size());
+    return (int)L.off.size();
 }
 
 // ---- OBU framing (host): sequence header, frame header, tile group; spec 5.5 (reduced still-picture sequence

@@ -258,6 +258,17 @@ int is_test_eval_mixed(is_handle *h, int form, int bit_depth, int n, const uint1
     return rc;
 }
 
+int is_test_code_symbols(is_handle *h, int n_tiles, const uint64_t *begin, const uint32_t *words, int qctx, uint8_t *out, uint64_t cap,
+                         uint64_t *off) {
+    if (!h || !begin || !words || !out || !off) return IS_ERR_INVALID;
+    IS_CK(cudaSetDevice(h->device));
+    std::string why;
+    const int rc = is::ent_test_code(n_tiles, begin, words, qctx, out, cap, off, &why);
+    return rc ? h->setErr(rc, "is_test_code_symbols: %s", why.c_str()) : IS_OK;
+}
+
+int is_test_cdfs(int qctx, uint16_t *cdf, size_t cap, uint16_t *off, uint8_t *n) { return is::ent_test_cdfs(qctx, cdf, cap, off, n); }
+
 int is_debug_analysis(is_handle *h, int bs, int64_t *J, uint8_t *cand, uint8_t *ncand, uint8_t *tx, uint16_t *tx_mask) {
     if (!h || !h->have || bs < 0 || bs >= 22) return IS_ERR_STATE;
     const FrameDesc &F = h->F;

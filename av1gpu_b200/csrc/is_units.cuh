@@ -68,6 +68,8 @@ cudaError_t ent_upload(const TableBlob &B);
 int ent_scratch(const is_ent_frame *frames, int n, uint64_t cap, size_t *bytes, std::string *err);
 int ent_launch(const is_ent_frame *frames, int n, uint64_t cap, void *scratch, size_t scratchBytes, cudaStream_t s, is_ent_out *out,
                uint32_t *frameTile0, std::string *err);
+int ent_test_code(int nTiles, const uint64_t *begin, const uint32_t *words, int qctx, uint8_t *out, uint64_t cap, uint64_t *off, std::string *err);
+int ent_test_cdfs(int qctx, uint16_t *cdf, size_t cap, uint16_t *off, uint8_t *n);
 int obu_assemble(const av1g_frame_params &fp, const uint8_t *payload, const uint64_t *off, uint32_t nTiles, std::vector<uint8_t> &o,
                  std::string *err);
 int avif_write(const av1g_frame_params &fp, const uint8_t *obu, size_t n, std::vector<uint8_t> &out, std::string *err);

@@ -57,7 +57,7 @@ class IsTimes(C.Structure):
 
 # every entry point declared in include/is_api.h
 EXPORTS = ["is_create", "is_destroy", "is_last_error", "is_build_info", "is_encode_device", "is_encode_host", "is_record_counts",
-           "is_record_copy", "is_record_device", "is_times_get", "is_test_fwd_quant", "is_test_eval_mixed", "is_test_inverse",
+           "is_record_copy", "is_record_device", "is_times_get", "is_test_fwd_quant", "is_test_eval_mixed", "is_test_code_symbols", "is_test_cdfs", "is_test_inverse",
            "is_test_predict", "is_debug_analysis", "is_debug_leaves", "is_debug_tables", "is_probe_int32", "is_set_trace", "is_get_trace",
            "is_fwd_quant_static", "is_encode_batch", "is_batch_counts", "is_batch_copy", "is_set_batch_options",
            "is_autotune_batch", "is_workspace_bytes", "is_workspace_bytes_format", "is_sl_create", "is_sl_destroy", "is_sl_set_params",
@@ -74,6 +74,15 @@ _lib = None
 def build_info():
     """Where the library's AV1 tables come from (is_build_info): "av1core headers <digest>, checkout" or ", headers only"."""
     return load_library().is_build_info().decode()
+
+
+def test_cdfs(qctx):
+    """The entries of av1g_cdfs at the start of a tile, and the CDFs' first entries and alphabets (no GPU needed)."""
+    L = load_library()
+    n = L.is_test_cdfs(qctx, None, 0, None, None)
+    cdf, off, alphabet = np.zeros(65536, np.uint16), np.zeros(n, np.uint16), np.zeros(n, np.uint8)
+    L.is_test_cdfs(qctx, cdf.ctypes.data, cdf.size, off.ctypes.data, alphabet.ctypes.data)
+    return cdf, off, alphabet
 
 
 def load_library():
@@ -98,6 +107,8 @@ def load_library():
     L.is_record_copy.argtypes = [vp, vp, vp, vp, vp, vp, vp * 3, vp]
     L.is_record_device.argtypes = [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), C.POINTER(vp)]
     L.is_times_get.argtypes = [vp, C.POINTER(IsTimes)]
+    L.is_test_code_symbols.argtypes = [vp, C.c_int, vp, vp, C.c_int, vp, C.c_uint64, vp]
+    L.is_test_cdfs.argtypes = [C.c_int, vp, C.c_size_t, vp, vp]
     L.is_test_eval_mixed.argtypes = [vp, C.c_int, C.c_int, C.c_int, vp, vp, C.c_int, vp, C.c_int, C.c_int, vp, vp, vp, vp, vp]
     L.is_test_fwd_quant.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, vp]
     L.is_test_inverse.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, C.c_int, vp, vp]
@@ -563,6 +574,15 @@ class Encoder:
                                               qindex, cx.ctypes.data, lv.ctypes.data, D.ctypes.data, R.ctypes.data, eob.ctypes.data),
                     "is_test_eval_mixed")
         return lv, D, R, eob
+
+    def test_code_symbols(self, tiles, qctx):
+        """Payloads of tiles given as arrays of symbol words (is_test_code_symbols)."""
+        begin = np.cumsum([0] + [len(t) for t in tiles]).astype(np.uint64)
+        w = np.ascontiguousarray(np.concatenate(tiles), np.uint32)
+        out, off = np.zeros(2 * len(w) + 64 * len(tiles), np.uint8), np.zeros(len(tiles) + 1, np.uint64)
+        self._check(self.L.is_test_code_symbols(self.h, len(tiles), begin.ctypes.data, w.ctypes.data, qctx, out.ctypes.data, out.size,
+                                                off.ctypes.data), "is_test_code_symbols")
+        return [out[int(a):int(b)].tobytes() for a, b in zip(off[:-1], off[1:])]
 
     def test_inverse(self, levels, tx_size, tx_type, qindex, w, h):
         levels = np.ascontiguousarray(levels, np.int16)

@@ -266,6 +266,13 @@ int is_test_fwd_quant(is_handle *h, int n, const int32_t *res, int tx_size, int 
 int is_test_eval_mixed(is_handle *h, int form, int bit_depth, int n, const uint16_t *src, const uint16_t *pred, int tx_size,
                        const uint8_t *tx_types, int plane, int qindex, const int32_t ctx[3], int16_t *levels, int64_t *D,
                        int64_t *R, int32_t *eob);
+/* The entropy coder alone: tiles of symbol words (begin [n_tiles + 1], words [begin[n_tiles]]; a word: kind 0 adaptive / 1
+ * equiprobable bit / 2, 3 split at the bottom / right frame edge | alphabet - 1 << 2 | symbol << 6 | CDF's entry in av1g_cdfs
+ * << 16) into payloads back to back, off [n_tiles + 1].  is_test_cdfs: the entries at the start of a tile, where each CDF
+ * begins and how many symbols it has (either may be NULL); returns the number of CDFs (no GPU needed). */
+int is_test_code_symbols(is_handle *h, int n_tiles, const uint64_t *begin, const uint32_t *words, int qctx, uint8_t *out,
+                         uint64_t cap, uint64_t *off);
+int is_test_cdfs(int qctx, uint16_t *cdf, size_t cap, uint16_t *off, uint8_t *n);
 /* Exact inverse transform (av1g_dequant + av1g_inv_txfm2d semantics) of n level blocks: res [n][H*W], flags [n]. */
 int is_test_inverse(is_handle *h, int n, const int16_t *levels, int tx_size, int tx_type, int qindex, int32_t *res,
                     uint32_t *flags);
