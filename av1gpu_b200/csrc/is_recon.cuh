@@ -847,7 +847,10 @@ __device__ void rc_leaf(const FrameDesc &F, RcWarp<Px, SS> &Wp, RcBig<Px> &Big, 
             sum = warp_sum(sum);
             cflAvg = (sum + (1 << (lw + lh - 1))) >> (lw + lh);
             __syncwarp();
-            // (a lane has at most 32 samples, |l| <= 8184 and |s - dc| <= 1023: its sums fit 32 bits)
+            // a lane has at most 32 of a CfL block's samples (32x32), |l| is at most 8 times the largest sample and |s - dc| at
+            // most it: the lanes' sums, and the squared errors of the whole block, fit 32 bits
+            constexpr long long top = (1 << BD) - 1;
+            static_assert(32 * (8 * top) * (8 * top) < (1ll << 31) && 1024 * top * top < (1ll << 31), "CfL sums need 64 bits");
             int num1 = 0, num2 = 0, den1 = 0;
 #pragma unroll 1
             for (int p = lane; p < W * H; p += 32) {
