@@ -18,8 +18,10 @@
 // coefficient.  In k_analysis_mid the levels stay in shared memory and the rate is coeff_bits over the scan positions: the
 // loop ends with the block's last level, and most blocks have few.  Both, with the slots' strides below: the analysis of a
 // 4000x3000 picture 70.0 -> 66.6 ms, 1920x1080 13.4 -> 11.8, 160x120 1.92 -> 1.66, the front end of 16 pictures of 256 to
-// 2048 samples a side with learned shortlists 128 -> 102 ms.  (On the 4000x3000 picture, whose blocks have few levels, contexts
-// looked up per coefficient in k_analysis_tiny take 2.3 ms less; on the batch they take 15 ms more.)
+// 2048 samples a side with learned shortlists 128 -> 102 ms.  k_analysis_tiny itself got slower on the 4000x3000 picture at
+// qindex 120, whose blocks have few levels (7.8 -> 9.1 ms alone; contexts looked up per coefficient would make the analysis 2.3 ms
+// less there and 15 ms more on the batch): which of the two a picture wants shows in its levels only, so there is no rule.
+// (Times with stand-in default CDFs in place of AV1's, as in is_k_ent.cu.)
 #pragma once
 #include "is_dev.cuh"
 #include "is_frame.cuh"
