@@ -45,7 +45,7 @@ UNITS = [("is_api.cu", "is_api.o", []),
          ("is_k_an.cu", "is_k_an10w.o", ["-DIS_BD=10", "-DIS_AN_PART=0"]), ("is_k_an.cu", "is_k_an10t.o", ["-DIS_BD=10", "-DIS_AN_PART=1"]),
          ("is_k_rc.cu", "is_k_rc8_420.o", ["-DIS_BD=8", "-DIS_SS=1"]), ("is_k_rc.cu", "is_k_rc8_444.o", ["-DIS_BD=8", "-DIS_SS=0"]),
          ("is_k_rc.cu", "is_k_rc10_420.o", ["-DIS_BD=10", "-DIS_SS=1"]), ("is_k_rc.cu", "is_k_rc10_444.o", ["-DIS_BD=10", "-DIS_SS=0"]),
-         ("is_k_ent.cu", "is_k_ent.o", []), ("is_k_pf.cu", "is_k_pf.o", [])]
+         ("is_k_ent.cu", "is_k_ent.o", []), ("is_k_pf.cu", "is_k_pf.o", []), ("is_k_test.cu", "is_k_test.o", [])]
 BUILD_DIR = os.path.join(HERE, "_build")
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills"]

@@ -308,87 +308,91 @@ bool packed_neighbours_match() {
     return true;
 }
 
+// the host-built tables of the units; an error where av1core's tables are not what the kernels were written for
+cudaError_t make_tables(TableBlob &B) {
+    const HostTables &T = host_tables();
+    B.cost.assign((size_t)4 * NCDF, 0);
+    for (int q = 0; q < 4; q++) memcpy(B.cost.data() + (size_t)q * NCDF, T.cost[q].data(), NCDF * 2);
+    memcpy(B.avgY, T.avgY, sizeof B.avgY);
+    memcpy(B.avgPart, T.avgPart, sizeof B.avgPart);
+    B.avgSkip0 = T.avgSkip0;
+    // scans packed per (tx size, class), one copy of each distinct table
+    std::vector<const uint16_t *> seen;
+    std::vector<uint16_t> seenOff;
+    for (int t = 0; t < 19; t++) {
+        const int n = std::min<int>(AV1G_T(Tx_Width)[t], 32) * std::min<int>(AV1G_T(Tx_Height)[t], 32);
+        const bool oneD = AV1G_T(Tx_Width)[t] <= 16 && AV1G_T(Tx_Height)[t] <= 16;
+        const int types[3] = {AV1G_DCT_DCT, AV1G_H_DCT, AV1G_V_DCT};   // class 2D, HORIZ, VERT
+        for (int c = 0; c < 3; c++) {
+            const uint16_t *sc = av1g_get_scan(t, (c == 0 || !oneD) ? AV1G_DCT_DCT : types[c]);
+            size_t k = 0;
+            while (k < seen.size() && seen[k] != sc) k++;
+            if (k == seen.size()) {
+                seen.push_back(sc);
+                seenOff.push_back((uint16_t)B.scanPack.size());
+                B.scanPack.insert(B.scanPack.end(), sc, sc + n);
+            }
+            B.scanOff[t][c] = seenOff[k];
+        }
+    }
+    cudaError_t e = cudaSuccess;
+    // the compile-time copies of spec tables in the per-thread search must equal av1core's
+    if (!packed_neighbours_match()) e = cudaErrorInvalidValue;
+    if (kDr23 != AV1G_T(Dr_Intra_Derivative)[23] || kDr45 != AV1G_T(Dr_Intra_Derivative)[45] || kDr67 != AV1G_T(Dr_Intra_Derivative)[67]) e = cudaErrorInvalidValue;
+    for (int lw = 2; lw <= 4; lw++)
+        for (int lh = 2; lw + lh <= 6; lh++)
+            for (int t = 0; t < 19; t++)
+                if (AV1G_T(Tx_Width_Log2)[t] == lw && AV1G_T(Tx_Height_Log2)[t] == lh && AV1G_T(Transform_Row_Shift)[t] != small_row_shift(lw, lh))
+                    e = cudaErrorInvalidValue;
+    // the analysis task lists and where each shape's tasks start in them
+    B.anTask = an_tasks(0);
+    B.anTaskBig = an_tasks(1);
+    auto starts = [](const std::vector<uint8_t> &t, int n, std::vector<int> &out) {
+        out.assign(n + 1, 0);
+        int k = 0;
+        for (size_t i = 0; i < t.size() / 3; i++)
+            if (i == 0 || t[3 * i] != t[3 * i - 3]) { if (k < n) out[k] = (int)i; k++; }
+        out[n] = (int)(t.size() / 3);
+        return k == n;
+    };
+    std::vector<int> stBig;
+    bool okShapes = starts(B.anTask, AN_SHAPES, B.anShapeStart) && starts(B.anTaskBig, ANB_SHAPES, stBig);
+    {   // the 64-sided list's groups: every shape of at least 2048 samples together, then one group per shape
+        B.anShapeStartBig.assign(ANB_GROUPS + 1, 0);
+        int g = 0;
+        B.anShapeStartBig[g++] = 0;
+        for (int k = 1; k < ANB_SHAPES && okShapes; k++) {
+            const int bs = B.anTaskBig[3 * stBig[k]];
+            if (AV1G_T(Num_4x4_Blocks_Wide)[bs] * AV1G_T(Num_4x4_Blocks_High)[bs] < 128) {
+                if (g >= ANB_GROUPS) okShapes = false;
+                else B.anShapeStartBig[g++] = stBig[k];
+            }
+        }
+        if (g != ANB_GROUPS) okShapes = false;
+        else B.anShapeStartBig[g] = stBig[ANB_SHAPES];
+    }
+    if (!okShapes) e = cudaErrorInvalidValue;
+    return e;
+}
+
 int upload_tables(int dev) {
     if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lk(g_upload_mu);
     if (g_uploaded[dev]) return 0;
-    {
-        const HostTables &T = host_tables();
-        TableBlob B;
-        B.cost.assign((size_t)4 * NCDF, 0);
-        for (int q = 0; q < 4; q++) memcpy(B.cost.data() + (size_t)q * NCDF, T.cost[q].data(), NCDF * 2);
-        memcpy(B.avgY, T.avgY, sizeof B.avgY);
-        memcpy(B.avgPart, T.avgPart, sizeof B.avgPart);
-        B.avgSkip0 = T.avgSkip0;
-        // scans packed per (tx size, class), one copy of each distinct table
-        std::vector<const uint16_t *> seen;
-        std::vector<uint16_t> seenOff;
-        for (int t = 0; t < 19; t++) {
-            const int n = std::min<int>(AV1G_T(Tx_Width)[t], 32) * std::min<int>(AV1G_T(Tx_Height)[t], 32);
-            const bool oneD = AV1G_T(Tx_Width)[t] <= 16 && AV1G_T(Tx_Height)[t] <= 16;
-            const int types[3] = {AV1G_DCT_DCT, AV1G_H_DCT, AV1G_V_DCT};   // class 2D, HORIZ, VERT
-            for (int c = 0; c < 3; c++) {
-                const uint16_t *sc = av1g_get_scan(t, (c == 0 || !oneD) ? AV1G_DCT_DCT : types[c]);
-                size_t k = 0;
-                while (k < seen.size() && seen[k] != sc) k++;
-                if (k == seen.size()) {
-                    seen.push_back(sc);
-                    seenOff.push_back((uint16_t)B.scanPack.size());
-                    B.scanPack.insert(B.scanPack.end(), sc, sc + n);
-                }
-                B.scanOff[t][c] = seenOff[k];
-            }
-        }
-        cudaError_t e = cudaSuccess;
-        // the compile-time copies of spec tables in the per-thread search must equal av1core's
-        if (!packed_neighbours_match()) e = cudaErrorInvalidValue;
-        if (kDr23 != AV1G_T(Dr_Intra_Derivative)[23] || kDr45 != AV1G_T(Dr_Intra_Derivative)[45] || kDr67 != AV1G_T(Dr_Intra_Derivative)[67]) e = cudaErrorInvalidValue;
-        for (int lw = 2; lw <= 4; lw++)
-            for (int lh = 2; lw + lh <= 6; lh++)
-                for (int t = 0; t < 19; t++)
-                    if (AV1G_T(Tx_Width_Log2)[t] == lw && AV1G_T(Tx_Height_Log2)[t] == lh && AV1G_T(Transform_Row_Shift)[t] != small_row_shift(lw, lh))
-                        e = cudaErrorInvalidValue;
-        // the analysis task lists and where each shape's tasks start in them
-        B.anTask = an_tasks(0);
-        B.anTaskBig = an_tasks(1);
-        auto starts = [](const std::vector<uint8_t> &t, int n, std::vector<int> &out) {
-            out.assign(n + 1, 0);
-            int k = 0;
-            for (size_t i = 0; i < t.size() / 3; i++)
-                if (i == 0 || t[3 * i] != t[3 * i - 3]) { if (k < n) out[k] = (int)i; k++; }
-            out[n] = (int)(t.size() / 3);
-            return k == n;
-        };
-        std::vector<int> stBig;
-        bool okShapes = starts(B.anTask, AN_SHAPES, B.anShapeStart) && starts(B.anTaskBig, ANB_SHAPES, stBig);
-        {   // the 64-sided list's groups: every shape of at least 2048 samples together, then one group per shape
-            B.anShapeStartBig.assign(ANB_GROUPS + 1, 0);
-            int g = 0;
-            B.anShapeStartBig[g++] = 0;
-            for (int k = 1; k < ANB_SHAPES && okShapes; k++) {
-                const int bs = B.anTaskBig[3 * stBig[k]];
-                if (AV1G_T(Num_4x4_Blocks_Wide)[bs] * AV1G_T(Num_4x4_Blocks_High)[bs] < 128) {
-                    if (g >= ANB_GROUPS) okShapes = false;
-                    else B.anShapeStartBig[g++] = stBig[k];
-                }
-            }
-            if (g != ANB_GROUPS) okShapes = false;
-            else B.anShapeStartBig[g] = stBig[ANB_SHAPES];
-        }
-        if (!okShapes) e = cudaErrorInvalidValue;
-        if (e == cudaSuccess) e = upload_common(B);
-        if (e == cudaSuccess) e = an_upload<8, 0>(B);
-        if (e == cudaSuccess) e = an_upload<8, 1>(B);
-        if (e == cudaSuccess) e = an_upload<10, 0>(B);
-        if (e == cudaSuccess) e = an_upload<10, 1>(B);
-        if (e == cudaSuccess) e = rc_upload<8, 1>(B);
-        if (e == cudaSuccess) e = rc_upload<8, 0>(B);
-        if (e == cudaSuccess) e = rc_upload<10, 1>(B);
-        if (e == cudaSuccess) e = rc_upload<10, 0>(B);
-        if (e == cudaSuccess) e = ent_upload(B);
-        g_uploaded[dev] = e == cudaSuccess;
-        return e == cudaSuccess ? 0 : (int)e;
-    }
+    TableBlob B;
+    cudaError_t e = make_tables(B);
+    if (e == cudaSuccess) e = upload_common(B);
+    if (e == cudaSuccess) e = an_upload<8, 0>(B);
+    if (e == cudaSuccess) e = an_upload<8, 1>(B);
+    if (e == cudaSuccess) e = an_upload<10, 0>(B);
+    if (e == cudaSuccess) e = an_upload<10, 1>(B);
+    if (e == cudaSuccess) e = rc_upload<8, 1>(B);
+    if (e == cudaSuccess) e = rc_upload<8, 0>(B);
+    if (e == cudaSuccess) e = rc_upload<10, 1>(B);
+    if (e == cudaSuccess) e = rc_upload<10, 0>(B);
+    if (e == cudaSuccess) e = ent_upload(B);
+    g_uploaded[dev] = e == cudaSuccess;
+    return e == cudaSuccess ? 0 : (int)e;
 }
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }

@@ -79,4 +79,10 @@ size_t pf_scratch_bytes(int W, int H, int bd, int c444);
 int pf_launch(const av1g_frame_params &fp, av1g_block *blocks, uint32_t nBlocks, const int8_t *sbCdefHost, uint8_t *const rec[3],
               const int rpitch[3], void *scratch, size_t scratchBytes, cudaStream_t s, std::string *err);
 
+// ---- test unit (is_k_test.cu): the small tx sizes' evaluations with a tx type per task; test_upload before the first call ----
+cudaError_t test_upload(const TableBlob &B);
+cudaError_t test_eval_mixed(int form, int bitDepth, int n, const uint16_t *src, const uint16_t *pred, int txSz, const uint8_t *types, int plane,
+                            int dcQ, int acQ, int qctx, int skipCtx, int dcCtx, int intraDir, int16_t *lv, long long *D, long long *R,
+                            int32_t *eob);
+
 }  // namespace is
